@@ -1,32 +1,31 @@
 // proj2d.cu -- 2D parallel-beam and fan-beam projector / backprojector.
 //
 // Forward (ParallelProjection2D / FanProjection2D): one thread per detector
-// pixel, blockIdx.y = view, blockIdx.z = batch element; the ray march follows
+// pixel, blockIdx.y = view, blockIdx.z = batch elements; the ray march follows
 // kernel_project2D (par_projector_2D_CudaKernel.cu.cc:28-102): box edges
 // index_to_physical(0|N) - 0.5 in mm, first sample at the entry with weight
 // 1/2, alpha advanced in a float, step 0.2 * min(spacing) mm, end correction
 // only when the sum is > 0, result scaled by |ray (.) spacing| (:141).
 // The reference samples a border/linear texture at index + 0.5; here the
-// same bilinear interpolation is done with exact FP32 weights.
+// same bilinear interpolation is done with exact FP32 weights.  The samples of
+// a ray that fall in one cell -- about four -- are summed in closed form
+// (sum_cells), at the march's own alphas, and slices of a batch that share
+// their geometry share the walk.  What bounds it: instruction issue, then the
+// L1 lines of the cell loads.
 // Given a workspace, the call first writes two copies of the batch as
-// bilinear CELLS -- cell (x, y) holds the four taps V(x + {0,1}, y + {0,1}),
-// with zeros outside the slice, for floors x, y in [-2, N] -- one x-fastest
-// and one y-fastest.  (The box starts half a millimetre below pixel 0: at
-// index -1 for 0.5 mm pixels, where rounding puts some rays' first sample a
-// hair below -1; the second border cell keeps every ray of such a view, and
-// so every lane of its warps, on the unclamped path.)  The cells hold FP32
-// taps for every storage type, so a sample is one 16-byte load with no bounds
-// tests and no widening.  A warp's 32 threads are 32 neighbouring detector pixels, so at each
-// step their samples lie along the detector direction: views whose rays run
-// mostly along y read the x-fastest cells, the others the y-fastest ones, so
-// the warp's loads stay on few cache lines.  Without a workspace the taps are
-// read from the caller's slice with a bounds test each.  Taps are combined in
-// the same order on every path, so the choice does not change a result.
-//
-// Launches with few rays (batch x views x detector pixels up to
-// SEG2D_MAX_RAYS) march each ray with SEG2D threads over contiguous ranges of
-// its samples, the range starts found in closed form on the same float alpha
-// sequence.
+// bilinear CELLS -- the cell of floors x, y in [-2, N] holds the four taps
+// V(x + {0,1}, y + {0,1}), with zeros outside the slice -- one x-fastest and one
+// y-fastest.  (The box starts half a millimetre below pixel 0: at index -1 for
+// 0.5 mm pixels, where rounding puts some rays' first sample a hair below -1;
+// the second border cell keeps every ray of such a view, and so every lane of
+// its warps, on the unclamped path.)  The cells hold FP32 taps for every
+// storage type, so a visit is one 16-byte load with no bounds tests and no
+// widening.  A warp's 32 threads are 32 neighbouring detector pixels, so their
+// cells lie along the detector direction: views whose rays run mostly along y
+// read the x-fastest cells, the others the y-fastest ones, so the warp's loads
+// stay on few cache lines.  Without a workspace the taps are read from the
+// caller's slice with a bounds test each.  Taps are combined in the same order
+// on every path, so the choice does not change a result.
 //
 // Backward (ParallelBackprojection2D / FanBackprojection2D): one thread per
 // pixel, loop over views, linear interpolation along the detector row;
@@ -43,349 +42,349 @@ namespace {
 
 constexpr float PI_REF = 3.14159265359f;  // par_backprojector_2D_CudaKernel.cu.cc:32
 constexpr int FP2_BLOCK = 128;
+
 constexpr int BP2_BLOCK_X = 32;
 constexpr int BP2_BLOCK_Y = 8;
 constexpr int BP2_CHUNK = BP2_BLOCK_X * BP2_BLOCK_Y;  // views per shared-memory table
 constexpr int BP2_VSPLIT = 4;                          // view groups of a small slice's backprojection
 constexpr long long BP2_SPLIT_MAX_PIXELS = 131072;     // pixels per launch up to which view groups are used
 
+// The forward walks a ray along its view's MAJOR axis m (the one its rays run
+// mostly along), the other being the minor axis n.  A bilinear cell holds the
+// four taps V(m0,n0), V(m1,n0), V(m0,n1), V(m1,n1), widened to FP32 whatever
+// the storage type (exact, so 16-bit storage gives the FP32 result of the
+// rounded input).  A source of taps is indexed by the floors (m, n) of a
+// sample and the slice s of the thread's slices.
+
+// From the caller's slices, taps outside them zero.
 template <typename T>
-__device__ __forceinline__ float interp2d_border(const T *__restrict__ img, float x, float y, int X, int Y)
+struct BorderTaps {
+    static constexpr bool ALIGN_COLUMNS = false;
+    const T *img;
+    size_t slice;
+    int s_m, s_n, M, N;  // element strides and extents of the axes
+    __device__ __forceinline__ float4 operator()(int m0, int n0, int s) const
+    {
+        const bool vm0 = (unsigned)m0 < (unsigned)M, vm1 = (unsigned)(m0 + 1) < (unsigned)M;
+        const bool vn0 = (unsigned)n0 < (unsigned)N, vn1 = (unsigned)(n0 + 1) < (unsigned)N;
+        const T *p = img + s * slice;
+        const int base = m0 * s_m + n0 * s_n;
+        float4 w;
+        w.x = (vm0 && vn0) ? load_as_float(p + base) : 0.0f;
+        w.y = (vm1 && vn0) ? load_as_float(p + base + s_m) : 0.0f;
+        w.z = (vm0 && vn1) ? load_as_float(p + base + s_n) : 0.0f;
+        w.w = (vm1 && vn1) ? load_as_float(p + base + s_m + s_n) : 0.0f;
+        return w;
+    }
+};
+
+// From a cell copy whose fast axis is n: columns of `pitch` cells, `slice`
+// cells per slice.  The copy holds floors in [-2, extent]; CLAMP takes others
+// to the nearest of these, whose taps are zero like theirs (for rays not
+// proven inside).
+template <bool CLAMP>
+struct CellTaps {
+    static constexpr bool ALIGN_COLUMNS = !CLAMP;
+    const float4 *cells;  // floor (-2, -2)
+    size_t slice;
+    unsigned pitch;
+    int M, N;
+    __device__ __forceinline__ float4 operator()(int m0, int n0, int s) const
+    {
+        if (CLAMP) m0 = min(max(m0, -2), M), n0 = min(max(n0, -2), N);
+        return __ldg(cells + s * slice + ((unsigned)m0 * pitch + (unsigned)n0 + 2u * (pitch + 1u)));
+    }
+};
+
+__device__ __forceinline__ float bilinear(const float4 &w, float tm, float tn)
 {
-    // sample positions stay inside the box (|x|, |y| << 2^22): exact FADD floor
-    const FloorFrac ffx = floor_frac(x), ffy = floor_frac(y);
-    const int x0 = ffx.i, y0 = ffy.i;
-    const float tx = ffx.f, ty = ffy.f;
-    const bool vx0 = (unsigned)x0 < (unsigned)X, vx1 = (unsigned)(x0 + 1) < (unsigned)X;
-    const bool vy0 = (unsigned)y0 < (unsigned)Y, vy1 = (unsigned)(y0 + 1) < (unsigned)Y;
-    const int base = y0 * X + x0;
-    const float p00 = (vy0 && vx0) ? load_as_float(img + base) : 0.0f;
-    const float p01 = (vy0 && vx1) ? load_as_float(img + base + 1) : 0.0f;
-    const float p10 = (vy1 && vx0) ? load_as_float(img + base + X) : 0.0f;
-    const float p11 = (vy1 && vx1) ? load_as_float(img + base + X + 1) : 0.0f;
-    const float p0 = lerp_ref(p00, p01, tx);
-    const float p1 = lerp_ref(p10, p11, tx);
-    return lerp_ref(p0, p1, ty);
+    return lerp_ref(lerp_ref(w.x, w.z, tn), lerp_ref(w.y, w.w, tn), tm);
 }
 
-template <typename T>
-struct BorderSampler {
-    const T *img;
-    int X, Y;
-    __device__ __forceinline__ float operator()(float x, float y) const { return interp2d_border<T>(img, x, y, X, Y); }
-};
-
-// The four taps of a bilinear cell in the order V(x0,y0), V(x1,y0),
-// V(x0,y1), V(x1,y1), widened to FP32 whatever the storage type: the
-// forward is bound by instruction issue, not by bytes (the slices' cells sit
-// in L2), and FP32 taps need no widening per sample (measured on the 64 x 512^2
-// fan batch: FP16 cells 43.7 ms, FP32 cells 42.3 ms per forward).  Widening is
-// exact, so 16-bit storage gives the FP32 result of the rounded input.
-struct Cell2 {
-    // the two x lerps of a cell: along y0 and along y1
-    __device__ static void xlerp(const float4 *c, float t, float &x0, float &x1)
-    {
-        const float4 w = __ldg(c);
-        x0 = lerp_ref(w.x, w.y, t), x1 = lerp_ref(w.z, w.w, t);
+// The alpha sequence a_0 = entry, a_{k+1} = fl(a_k + step) of kernel_project2D
+// (par_projector_2D_CudaKernel.cu.cc:58-102) in closed form over runs of equal
+// increments: inside the binade [2^e, 2^(e+1)) of a, a = M u with u = 2^(e-23)
+// and M in [2^23, 2^24), every exact sum a_k + step lies at the same offset
+// from the grid of multiples of u, so each step adds D u with D = round(step /
+// u); a result equal to 2^(e+1) (M = 2^24) is also right (the sum lies within
+// u/2 of it on either side's grid).  A sum halfway between two grid values
+// goes to the even one, so from an even M on the increment is the even one of
+// the two neighbours of step / u.
+// Given a sample at a < am, returns n >= 1 samples a + j delta, j < n, all of
+// them below am, n <= kmax, and their successor a_{n} in `next`.  Where the
+// closed form does not hold (a not positive normal, the step past a binade),
+// n = 1.  n stays below 2^22, so j is exact in FP32.
+__device__ __forceinline__ int alpha_run(float a, float am, float step, int kmax, float &delta, float &next)
+{
+    delta = 0.0f;
+    next = __fadd_rn(a, step);
+    const int sb = __float_as_int(step), se = (sb >> 23) & 0xff;
+    const int bits = __float_as_int(a), be = (bits >> 23) & 0xff;
+    if (bits <= 0 || be <= 23 || be == 0xff || sb <= 0 || se == 0 || se == 0xff) return 1;  // (u normal too)
+    const unsigned ms = (unsigned)(sb & 0x7fffff) | 0x800000u;
+    const unsigned M = (unsigned)(bits & 0x7fffff) | 0x800000u;
+    // D = round(step / u), step / u = ms 2^(se - be)
+    const int sh = be - se;
+    unsigned D;
+    if (sh < 0) {
+        return 1;  // step >= 2^24 u: no second sample in the binade
+    } else if (sh == 0) {
+        D = ms;
+    } else if (sh >= 25) {
+        D = 0u;  // step below u / 2: the sequence stalls at a
+    } else {
+        const unsigned rem = ms & ((1u << sh) - 1u), half = 1u << (sh - 1);
+        D = ms >> sh;
+        if (rem == half) {
+            if (M & 1u) return 1;
+            D += D & 1u;
+        } else {
+            D += rem > half ? 1u : 0u;
+        }
     }
-    __device__ static float4 make(float a, float b, float c, float d) { return make_float4(a, b, c, d); }
-};
-
-// Bilinear interpolation from a cell copy; `origin` is the cell of floor
-// (0, 0), (s_x, s_y) the cell strides.  Floors must lie in [-2, N].
-struct CellSampler2 {
-    const float4 *origin;
-    unsigned s_x, s_y;
-    unsigned bias;  // -FLOOR_BIAS * (s_x + s_y), modulo 2^32: the floors' bias folded into one offset
-
-    __device__ CellSampler2(const float4 *o, int sx, int sy)
-        : origin(o), s_x((unsigned)sx), s_y((unsigned)sy), bias(0u - (unsigned)FLOOR_BIAS * ((unsigned)sx + (unsigned)sy))
-    {
+    unsigned n = min((unsigned)kmax, 1u << 22);
+    if (D > 0u) {
+        // results a + j D u stay on this grid while M + j D <= 2^24
+        n = min(n, (0x1000000u - M) / D);
+        if (n == 0u) return 1;
+        // and the march stops at the first alpha not below am (am > a, so its
+        // binade is e or above; two or more above, it is out of reach)
+        const int amb = __float_as_int(am), ae = (amb >> 23) & 0xff;
+        if (ae - be <= 1) {
+            const unsigned am_u = ((unsigned)(amb & 0x7fffff) | 0x800000u) << (ae - be);  // am / u, exact
+            n = min(n, (am_u - M + D - 1u) / D);
+        }
     }
+    delta = (float)D * __int_as_float((be - 23) << 23);               // D u, exact: D <= 2^24
+    next = __int_as_float((be << 23) + (int)(M + n * D) - 0x800000);  // M + n D = 2^24 gives 2^(e+1)
+    return (int)n;
+}
 
-    __device__ __forceinline__ float operator()(float x, float y) const
-    {
-        const FloorFrac fx = floor_frac(x), fy = floor_frac(y);
-        const unsigned idx = (unsigned)fx.bits * s_x + (unsigned)fy.bits * s_y + bias;
-        float x0, x1;
-        Cell2::xlerp(origin + (int)idx, fx.f, x0, x1);
-        return lerp_ref(x0, x1, fy.f);
-    }
-};
-
-// For rays whose march leaves [-1.5, N + 0.5]: positions clamped into it,
-// which changes no tap weight that is not zero either way.
-struct ClampedCellSampler2 {
-    CellSampler2 s;
-    float xmax, ymax;
-    __device__ __forceinline__ float operator()(float x, float y) const
-    {
-        return s(fminf(fmaxf(x, -1.5f), xmax), fminf(fmaxf(y, -1.5f), ymax));
-    }
-};
-
-// The iteration bound of march2d's loops.
+// The iteration bound of the march.
 __device__ __forceinline__ int march2d_max_iter(float a, float am, float step)
 {
     const double bound = ((double)am - (double)a) / (double)step + 4.0;
     return bound > 1.0e8 ? 100000000 : (int)bound;
 }
 
-// The ray march of kernel_project2D (par_projector_2D_CudaKernel.cu.cc:58-102)
-// at positions (bx + a gx, by + a gy) in index space, eight (then four, two,
-// one) samples per iteration (their gathers overlap) with the same alpha
-// sequence and order of additions as one at a time.
-template <typename F>
-__device__ __forceinline__ float march2d(float a, float am, float step, float gx, float bx, float gy, float by,
-                                         const F &sample)
+// A ray through index space: position (bm + a gm, bn + a gn) at alpha a.
+struct Ray2D {
+    float a, am, step, gm, bm, gn, bn;
+    __device__ __forceinline__ float m(float al) const { return fmaf(al, gm, bm); }
+    __device__ __forceinline__ float n(float al) const { return fmaf(al, gn, bn); }
+};
+
+// A pair of values on the packed FP32 instructions (m in .x, n in .y): each
+// costs one issue slot for both halves, and the kernel is bound by issue.
+__device__ __forceinline__ float2 pair(float a, float b) { return make_float2(a, b); }
+
+struct FloorFrac2 {
+    int mi, ni;
+    float2 f;
+};
+// floor_frac (common.cuh) of both halves
+__device__ __forceinline__ FloorFrac2 floor_frac2(float2 x)
 {
-    const int max_iter = march2d_max_iter(a, am, step);
-    float pixel = 0.0f, px = 0.0f, py = 0.0f;
-    int iter = 0;
-    if (a < am) {
-        px = fmaf(a, gx, bx);
-        py = fmaf(a, gy, by);
-        pixel += 0.5f * sample(px, py);
-        a += step;
-        ++iter;
-    }
-    // eight samples per compare while the eighth alpha is still before the exit
-    while (iter + 7 < max_iter) {
-        const float a1 = a + step, a2 = a1 + step, a3 = a2 + step, a4 = a3 + step, a5 = a4 + step, a6 = a5 + step,
-                    a7 = a6 + step;
-        if (!(a7 < am)) break;
-        const float v0 = sample(fmaf(a, gx, bx), fmaf(a, gy, by));
-        const float v1 = sample(fmaf(a1, gx, bx), fmaf(a1, gy, by));
-        const float v2 = sample(fmaf(a2, gx, bx), fmaf(a2, gy, by));
-        const float v3 = sample(fmaf(a3, gx, bx), fmaf(a3, gy, by));
-        const float v4 = sample(fmaf(a4, gx, bx), fmaf(a4, gy, by));
-        const float v5 = sample(fmaf(a5, gx, bx), fmaf(a5, gy, by));
-        const float v6 = sample(fmaf(a6, gx, bx), fmaf(a6, gy, by));
-        px = fmaf(a7, gx, bx);
-        py = fmaf(a7, gy, by);
-        const float v7 = sample(px, py);
-        pixel += v0;
-        pixel += v1;
-        pixel += v2;
-        pixel += v3;
-        pixel += v4;
-        pixel += v5;
-        pixel += v6;
-        pixel += v7;
-        a = a7 + step;
-        iter += 8;
-    }
-    // four samples per compare while the fourth alpha is still before the
-    // exit (the sequence never decreases, so the first three are too)
-    while (iter + 3 < max_iter) {
-        const float a1 = a + step, a2 = a1 + step, a3 = a2 + step;
-        if (!(a3 < am)) break;
-        const float v0 = sample(fmaf(a, gx, bx), fmaf(a, gy, by));
-        const float v1 = sample(fmaf(a1, gx, bx), fmaf(a1, gy, by));
-        const float v2 = sample(fmaf(a2, gx, bx), fmaf(a2, gy, by));
-        px = fmaf(a3, gx, bx);
-        py = fmaf(a3, gy, by);
-        const float v3 = sample(px, py);
-        pixel += v0;
-        pixel += v1;
-        pixel += v2;
-        pixel += v3;
-        a = a3 + step;
-        iter += 4;
-    }
-    while (a < am && iter < max_iter) {
-        const float a1 = a + step;
-        if (a1 < am && iter + 1 < max_iter) {
-            const float qx = fmaf(a, gx, bx), qy = fmaf(a, gy, by);
-            px = fmaf(a1, gx, bx);
-            py = fmaf(a1, gy, by);
-            const float v0 = sample(qx, qy);
-            const float v1 = sample(px, py);
-            pixel += v0;
-            pixel += v1;
-            a = a1 + step;
-            iter += 2;
-        } else {
-            px = fmaf(a, gx, bx);
-            py = fmaf(a, gy, by);
-            pixel += sample(px, py);
-            a += step;
-            ++iter;
-        }
-    }
-    pixel *= step;
-    if (pixel > 0.0f) {  // :88-100
-        const float last_val = sample(px, py);
-        pixel -= 0.5f * step * last_val;
-        a -= step;
-        const float last_step = am - a;
-        pixel += 0.5f * last_step * last_val;
-        px = fmaf(am, gx, bx);
-        py = fmaf(am, gy, by);
-        pixel += 0.5f * last_step * sample(px, py);
-    }
-    return pixel;
+    const float magic = 12582912.0f;
+    const float2 y = __fadd2_rd(x, pair(magic, magic));
+    FloorFrac2 r;
+    r.mi = __float_as_int(y.x) - FLOOR_BIAS;
+    r.ni = __float_as_int(y.y) - FLOOR_BIAS;
+    r.f = __ffma2_rn(__fadd2_rn(y, pair(-magic, -magic)), pair(-1.0f, -1.0f), x);
+    return r;
 }
 
-// Ray segments.  A launch with few rays (one 256^2 slice scanned over 180
-// views by 367 pixels has 66 k) fills a fraction of the GPU's warp slots
-// while each thread marches ~1800 samples in sequence.  Its rays are marched
-// by SEG2D threads each, over contiguous ranges of the ray's samples; the
-// ranges start at alphas found in closed form (alpha_advance), so every
-// sample sits where the one-thread march puts it, and the block adds the
-// ranges' sums in order before the end correction (a different order of FP32
-// additions than one thread's: the results differ in the last bits).  A full
-// launch does better with one thread per ray (measured on 256 such slices per
-// call: 14.1 ms per forward against 17.4 ms with segments), so segments are
-// used up to SEG2D_MAX_RAYS rays per launch (batch x views x pixels).
+// A linear run of samples: the coordinates c0 + j d at sample j, and the
+// number of samples from a fraction f to the cell's far faces, r0 - f inv
+// (ninv = -inv).
+struct Run2D {
+    float2 c0, d, ninv, r0;
+    __device__ __forceinline__ static void face(float d, float &ninv, float &r0)
+    {
+        const bool moves = fabsf(d) > 1.0e-30f;
+        const float inv = moves ? __frcp_rn(d) : 0.0f;
+        ninv = -inv;
+        r0 = !moves ? 1.0e30f : (d > 0.0f ? inv : 0.0f);
+    }
+    __device__ __forceinline__ void set(const Ray2D &ray, float a, float delta)
+    {
+        c0 = pair(ray.m(a), ray.n(a));
+        d = pair(delta * ray.gm, delta * ray.gn);
+        face(d.x, ninv.x, r0.x);
+        face(d.y, ninv.y, r0.y);
+    }
+    __device__ __forceinline__ FloorFrac2 at(float j) const { return floor_frac2(__ffma2_rn(pair(j, j), d, c0)); }
+};
+
+// The sums of `kmax` (or all) samples of the ray from alpha `a` on, for NS
+// slices: samples at the march's own alphas, one cell visit at a time.  The
+// step is a fifth of a pixel, so a ray takes about four samples per cell, and
+// inside a cell the interpolant along the ray is a quadratic in the sample
+// number: the L samples of a visit add up to L times the interpolant at their
+// middle plus the cross term's spread, C dm dn L (L^2 - 1) / 12 with C the
+// cell's mixed difference.  (The interpolant is continuous across cell faces:
+// a sample within rounding of a face may go to either cell.)  Returns the
+// alpha after the last sample and the last sample's alpha in `a_last`.
+//
+// ALIGN_COLUMNS: the lanes of `mask` (neighbouring rays) walk the columns of
+// the major axis together, a few (COLS) at a time -- a lane visits cells only up
+// to the warp's common column, counted from the first lane's entry -- so a
+// warp's loads fall on few columns, at neighbouring n.  Free-running lanes
+// spread over as many columns as lines (10 L1 cycles per load, the L1 98 %
+// busy); strict alignment (COLS = 1) idles lanes whose neighbours cross more
+// rows.  64 fan slices of 512^2, four per thread: 21.7 ms free-running, 17.0 /
+// 14.4 / 13.5 / 13.2 / 13.5 ms for COLS = 1 / 2 / 4 / 8 / 16; with one slice per
+// thread 16 is best.
+template <int NS, typename Taps>
+__device__ __forceinline__ float sum_cells(const Ray2D &ray, float a, int kmax, const Taps &taps, unsigned mask,
+                                           float (&acc)[NS], float &a_last)
+{
+    constexpr int COLS = NS == 1 ? 16 : 8;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) acc[s] = 0.0f;
+    Run2D run;
+    float nf, jf, spread0, next = a;
+    bool alive;
+    auto next_run = [&]() {  // the next run of equal increments (one to three per ray)
+        a = next;
+        alive = a < ray.am && kmax > 0;
+        if (!alive) return;
+        float delta;
+        const int n = alpha_run(a, ray.am, ray.step, kmax, delta, next);
+        kmax -= n;
+        nf = (float)n;
+        jf = 0.0f;
+        run.set(ray, a, delta);
+        spread0 = run.d.x * run.d.y * (1.0f / 12.0f);
+        a_last = fmaf(nf - 1.0f, delta, a);  // exact: a value of the sequence
+    };
+    a_last = a;
+    next_run();
+    FloorFrac2 p = floor_frac2(pair(ray.m(a), ray.n(a)));
+    // the lane's column: the floor along m in the ray's direction, relative
+    // to the first lane's entry
+    int sign = 0, off = 0;
+    if (Taps::ALIGN_COLUMNS) {
+        sign = ray.gm < 0.0f ? -1 : 1;
+        off = -__reduce_min_sync(mask, alive ? sign * p.mi : 0x7fffffff);
+    }
+    for (int column = COLS - 1; alive; column += COLS) {
+        while (alive && (!Taps::ALIGN_COLUMNS || sign * p.mi + off <= column)) {
+            float4 w[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) w[s] = taps(p.mi, p.ni, s);
+            // samples of this visit: up to the nearer face or the run's end,
+            // at least one (ceiling by a sum rounded up, as floor_frac's;
+            // exact below 2^22, and nf is)
+            const float2 r = __ffma2_rn(p.f, run.ninv, run.r0);
+            const float c = fminf(fminf(r.x, r.y), nf - jf);
+            const float L = fmaxf(__fadd_rn(__fadd_ru(c, 12582912.0f), -12582912.0f), 1.0f);
+            const float h = fmaf(L, 0.5f, -0.5f);
+            const float2 mid = __ffma2_rn(pair(h, h), run.d, p.f);
+            const float spread = fmaf(L, L, -1.0f) * spread0;
+            jf += L;
+            if (jf >= nf) next_run();
+            p = run.at(jf);
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                const float2 lo = pair(w[s].x, w[s].y), hi = pair(w[s].z, w[s].w);
+                const float2 dn = __ffma2_rn(lo, pair(-1.0f, -1.0f), hi);
+                const float2 q = __ffma2_rn(pair(mid.y, mid.y), dn, lo);
+                const float v = fmaf(dn.y - dn.x, spread, fmaf(mid.x, q.y - q.x, q.x));
+                acc[s] = fmaf(L, v, acc[s]);
+            }
+        }
+    }
+    return a;
+}
+
+// Ray segments.  A launch with few rays fills a fraction of the GPU's warp
+// slots while each thread walks some hundred cells in sequence.  Its rays are
+// marched by SEG2D threads each, one per band of columns along the major axis
+// (so the lanes of a warp, neighbouring rays, stay on common columns), and the
+// block adds the bands' sums in order before the end correction (a different
+// order of FP32 additions than one thread's: the results differ in the last
+// bits).  Used up to SEG2D_MAX_RAYS rays per launch (batch x views x pixels), or
+// SEG2D_MAX_RAYS_SHARED where the slices of a batch share their geometry and a
+// thread can take several: measured per call, segments / one thread per ray,
+// 256^2 parallel slices, 66 k rays 0.139 / 0.191 ms, 132 k (two slices) 0.187 /
+// 0.204, 198 k (three) 0.238 / 0.221; one 387 x 451 fan slice (234 k) 0.348 /
+// 0.384, one 512^2 fan slice (369 k) 0.555 / 0.551.
 constexpr int SEG2D = 4;
-constexpr long long SEG2D_MAX_RAYS = 150000;
+constexpr long long SEG2D_MAX_RAYS = 300000, SEG2D_MAX_RAYS_SHARED = 150000;
 
-// The alpha sequence of march2d: a_{k+1} = fl(a_k + step).  Moves (a, k)
-// forward while k < kmax and a < am, as the one-at-a-time loop does, in
-// closed form over runs of equal increments, in integer arithmetic on the
-// floats' significands: inside the binade [2^e, 2^(e+1)) of a, a = M u with
-// u = 2^(e-23) and M in [2^23, 2^24), every exact sum a_k + step lies at the
-// same offset from the grid of multiples of u, so each step adds D u with
-// D = round(step / u); a result equal to 2^(e+1) (M = 2^24) is also right
-// (the sum lies within u/2 of it on either side's grid), and the step past it
-// is one float addition.  Returns false -- sequence not followed -- for a or
-// step not positive normal, a step below u/2 (the loop stalls) or a sum
-// halfway between two grid values (round-to-even then alternates).
-__device__ bool alpha_advance(float &a, int &k, int kmax, float am, float step)
+// The number of the ray's samples at alphas below `limit`, at most kmax, and
+// the alpha that follows them.
+__device__ __forceinline__ int samples_before(const Ray2D &ray, float limit, int kmax, float &a)
 {
-    const int sb = __float_as_int(step), se = (sb >> 23) & 0xff;
-    if (sb <= 0 || se == 0 || se == 0xff) return false;
-    const unsigned ms = (unsigned)(sb & 0x7fffff) | 0x800000u;
-    const int amb = __float_as_int(am), ae = (amb >> 23) & 0xff;
-    for (int guard = 0; guard < 512 && k < kmax && a < am; ++guard) {
-        const int bits = __float_as_int(a), be = (bits >> 23) & 0xff;
-        if (bits <= 0 || be == 0 || be == 0xff) return false;
-        const unsigned M = (unsigned)(bits & 0x7fffff) | 0x800000u;
-        // D = round(step / u), step / u = ms 2^(se - be)
-        const int sh = be - se;
-        unsigned D;
-        if (sh <= 0) {
-            D = -sh >= 8 ? 0x2000000u : ms << -sh;
-        } else {
-            if (sh >= 26) return false;
-            const unsigned rem = ms & ((1u << sh) - 1u), half = 1u << (sh - 1);
-            if (rem == half) return false;
-            D = (ms >> sh) + (rem > half ? 1u : 0u);
-            if (D == 0u) return false;
-        }
-        // results a + j D u, j = 1..m, stay on this grid (M + j D <= 2^24)
-        unsigned m = D > 0x1000000u ? 0u : (0x1000000u - M) / D;
-        if (m == 0u) {
-            a = __fadd_rn(a, step);
-            ++k;
-            continue;
-        }
-        // and the loop stops after the step from the last alpha below am
-        // (am > a, so its binade is e or above; two or more above, it is out of reach)
-        if (ae - be <= 1) {
-            const unsigned am_u = ((unsigned)(amb & 0x7fffff) | 0x800000u) << (ae - be);  // am / u, exact
-            m = min(m, (am_u - M + D - 1u) / D);
-        }
-        m = min(m, (unsigned)(kmax - k));
-        a = __int_as_float((be << 23) + (int)(M + m * D) - 0x800000);  // M + m D = 2^24 gives 2^(e+1)
-        k += (int)m;
-    }
-    return k >= kmax || !(a < am);
-}
-
-// Samples k0 .. k1 - 1 of march2d's ray, a = a_{k0} on entry and a_{k1} on
-// return (the same float additions); sample 0 weighs 1/2.  Returns their sum
-// in order and the last one's value in `last`.
-template <typename F>
-__device__ __forceinline__ float march2d_range(float &a, int k0, int k1, float step, float gx, float bx, float gy,
-                                               float by, const F &sample, float &last)
-{
-    float sum = 0.0f;
-    int k = k0;
-    if (k == 0 && k < k1) {
-        last = sample(fmaf(a, gx, bx), fmaf(a, gy, by));
-        sum += 0.5f * last;
-        a += step;
-        ++k;
-    }
-    for (; k + 8 <= k1; k += 8) {
-        const float a1 = a + step, a2 = a1 + step, a3 = a2 + step, a4 = a3 + step, a5 = a4 + step, a6 = a5 + step,
-                    a7 = a6 + step;
-        const float v0 = sample(fmaf(a, gx, bx), fmaf(a, gy, by));
-        const float v1 = sample(fmaf(a1, gx, bx), fmaf(a1, gy, by));
-        const float v2 = sample(fmaf(a2, gx, bx), fmaf(a2, gy, by));
-        const float v3 = sample(fmaf(a3, gx, bx), fmaf(a3, gy, by));
-        const float v4 = sample(fmaf(a4, gx, bx), fmaf(a4, gy, by));
-        const float v5 = sample(fmaf(a5, gx, bx), fmaf(a5, gy, by));
-        const float v6 = sample(fmaf(a6, gx, bx), fmaf(a6, gy, by));
-        const float v7 = sample(fmaf(a7, gx, bx), fmaf(a7, gy, by));
-        sum += v0;
-        sum += v1;
-        sum += v2;
-        sum += v3;
-        sum += v4;
-        sum += v5;
-        sum += v6;
-        sum += v7;
-        last = v7;
-        a = a7 + step;
-    }
-    for (; k < k1; ++k) {
-        last = sample(fmaf(a, gx, bx), fmaf(a, gy, by));
-        sum += last;
-        a += step;
-    }
-    return sum;
-}
-
-// One ray: SEG = 1, march2d's pixel.  SEG > 1: the sum of range `seg` of
-// the ray's samples (n samples, counted by alpha_advance); the range holding
-// the last sample also returns that sample's value, the value at the exit and
-// the end correction's last step (am - fl(a_n - step), as march2d forms it).
-// A sequence alpha_advance cannot follow is marched whole by range 0 (`whole`).
-template <int SEG, typename F>
-__device__ __forceinline__ float march_ray(float a, float am, float step, float gx, float bx, float gy, float by,
-                                           const F &sample, int seg, float &last, float &end_val, float &last_step,
-                                           bool &holds_last, bool &whole)
-{
-    if (SEG == 1) return march2d(a, am, step, gx, bx, gy, by, sample);
-    float an = a;
     int n = 0;
-    if (!alpha_advance(an, n, march2d_max_iter(a, am, step), am, step)) {
-        whole = true;
-        return seg == 0 ? march2d(a, am, step, gx, bx, gy, by, sample) : 0.0f;
-    }
-    const int k0 = (int)((long long)seg * n / SEG), k1 = (int)((long long)(seg + 1) * n / SEG);
-    int k = 0;
-    alpha_advance(a, k, k0, am, step);  // every alpha before k0 <= n - 1 is below am
-    const float sum = march2d_range(a, k0, k1, step, gx, bx, gy, by, sample, last);
-    if (k1 == n && k1 > k0) {
-        holds_last = true;
-        last_step = am - (a - step);
-        end_val = sample(fmaf(am, gx, bx), fmaf(am, gy, by));
-    }
-    return sum;
+    float delta, next;
+    a = ray.a;
+    for (; a < limit && n < kmax; a = next) n += alpha_run(a, limit, ray.step, kmax - n, delta, next);
+    return n;
 }
 
-// SEG = 1: one thread per detector pixel.  SEG > 1: FP2_BLOCK / SEG pixels
-// per block, warp w of the block marching range w of their rays.
-template <typename T, typename Tout, bool FAN, int SEG>
-// (12 blocks per SM: 40 registers hold the eight-sample loop; the kernel is
-// bound by the cell loads' latency, so more resident warps pay.  SEG > 1
-// keeps a range's bookkeeping across the loop: 10 blocks, 48 registers.)
-__global__ void __launch_bounds__(FP2_BLOCK, SEG == 1 ? 12 : 10)
+// The sums of one ray's samples, sample 0 with weight 1/2 (SEG > 1: those of
+// band `seg` of the `extent` columns), and for the thread that holds the last
+// sample its value, the value at the exit and the end correction's last step
+// (am - fl(a_n - step)).
+template <int SEG, int NS, typename Taps>
+__device__ __forceinline__ void march_ray(const Ray2D &ray, const Taps &taps, unsigned mask, int seg, int extent,
+                                          float (&sum)[NS], float (&last)[NS], float (&end_val)[NS],
+                                          float &last_step, bool &holds_last)
+{
+    int kmax = march2d_max_iter(ray.a, ray.am, ray.step), k0 = 0;
+    float a = ray.a;
+    if (SEG > 1) {
+        float b;
+        const int n = samples_before(ray, ray.am, kmax, b);
+        // band boundaries in the ray's direction; neighbouring bands evaluate
+        // the same bound, so every sample falls in one band (a bound that is
+        // not a number, or behind the ray, leaves the earlier band empty)
+        auto bound = [&](int i) {
+            const float m = (float)extent * ((float)(ray.gm < 0.0f ? SEG - i : i) / (float)SEG);
+            return fminf((m - ray.bm) / ray.gm, ray.am);
+        };
+        int k1 = n;
+        if (seg > 0) k0 = samples_before(ray, bound(seg), kmax, a);
+        if (seg < SEG - 1) k1 = samples_before(ray, bound(seg + 1), kmax, b);
+        kmax = max(k1 - k0, 0);
+        holds_last = kmax > 0 && k1 == n;
+    } else {
+        holds_last = a < ray.am && kmax > 0;
+    }
+    float a_last;
+    const float a_end = sum_cells<NS>(ray, a, kmax, taps, mask, sum, a_last);
+    auto sample = [&](float al, int s) {
+        const FloorFrac fm = floor_frac(ray.m(al)), fn = floor_frac(ray.n(al));
+        return bilinear(taps(fm.i, fn.i, s), fm.f, fn.f);
+    };
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        if (k0 == 0 && kmax > 0 && a < ray.am) sum[s] -= 0.5f * sample(a, s);
+        if (holds_last) last[s] = sample(a_last, s), end_val[s] = sample(ray.am, s);
+    }
+    if (holds_last) last_step = ray.am - (a_end - ray.step);
+}
+
+// SEG = 1: one thread per detector pixel and NS slices (NS > 1: slices that
+// share the geometry).  SEG > 1: FP2_BLOCK / SEG pixels per block, warp w of
+// the block marching range w of their rays.
+template <typename T, typename Tout, bool FAN, int SEG, int NS>
+// (8 blocks per SM, 64 registers, hold the walk; four slices need 72.  More
+// or fewer resident blocks measured within 1 to 5 % slower.)
+__global__ void __launch_bounds__(FP2_BLOCK, NS == 4 ? 7 : 8)
     projection2d_kernel(const T *__restrict__ vol, const float4 *__restrict__ cells_x,
                         const float4 *__restrict__ cells_y, Tout *__restrict__ sino, Geom2D geo,
-                        int X, int Y, int W, int n_proj, int geom_batch)
+                        int X, int Y, int W, int n_proj, int batch, int geom_batch)
 {
     constexpr int RAYS = FP2_BLOCK / SEG;  // rays per block
     static_assert(SEG == 1 || RAYS == 32, "a segment per warp");
+    static_assert(SEG == 1 || NS == 1, "ranges take one slice");
     const int lane = threadIdx.x % RAYS, seg = threadIdx.x / RAYS;
     const int u = blockIdx.x * RAYS + lane;
     const int p = blockIdx.y;
-    const int b = blockIdx.z;
-    if (SEG == 1 && u >= W) return;
+    const int b = blockIdx.z * NS;
     const bool live = u < W;
     const int g = geom_batch == 1 ? 0 : b;
     const float sx = geo.volume_spacing[2 * g + 1], sy = geo.volume_spacing[2 * g + 0];
@@ -439,65 +438,73 @@ __global__ void __launch_bounds__(FP2_BLOCK, SEG == 1 ? 12 : 10)
         amax = fmin(amax, fmax(a0, a1));
     }
 
-    const float step = 0.2f * fminf(sx, sy);
+    Ray2D ray;
+    ray.step = 0.2f * fminf(sx, sy);
     const float dx = (float)rx, dy = (float)ry;
-    float pixel = 0.0f;                 // SEG > 1: this range's sum (or the whole ray's pixel, `whole`)
-    float last = 0.0f, end_val = 0.0f;  // SEG > 1, the range holding the last sample: its value and
-    float last_step = 0.0f;             // the end correction's sample and step
-    bool holds_last = false, whole = false;
-    if (live && step > 0.0f && amin < amax) {
-        // sample positions in index space: idx = (src + a r - o) / s
-        const float isx = 1.0f / sx, isy = 1.0f / sy;
-        const float bx = (float)((srcx - ox) / sx), by = (float)((srcy - oy) / sy);
-        const float gx = dx * isx, gy = dy * isy;
-        const float a = (float)amin, am = (float)amax;
-        if (cells_x) {
-            // block-uniform layout choice: y-fastest cells when the view's
-            // rays run mostly along x (fan: the central ray)
-            const bool fast_y = fabsf(ray_in.x) > fabsf(ray_in.y);
-            const size_t slice = (size_t)(X + 3) * (Y + 3);
-            const CellSampler2 cs = fast_y ? CellSampler2(cells_y + b * slice + 2 * (Y + 3) + 2, Y + 3, 1)
-                                           : CellSampler2(cells_x + b * slice + 2 * (X + 3) + 2, 1, X + 3);
-            // every position of the march lies between its two end points
-            const float x0 = fmaf(a, gx, bx), y0 = fmaf(a, gy, by), x1 = fmaf(am, gx, bx), y1 = fmaf(am, gy, by);
-            const float xmax = (float)X + 0.5f, ymax = (float)Y + 0.5f;
-            const bool inside = fminf(x0, x1) >= -1.5f && fminf(y0, y1) >= -1.5f && fmaxf(x0, x1) <= xmax &&
-                                fmaxf(y0, y1) <= ymax;
-            if (inside)
-                pixel = march_ray<SEG>(a, am, step, gx, bx, gy, by, cs, seg, last, end_val, last_step, holds_last,
-                                       whole);
-            else
-                pixel = march_ray<SEG>(a, am, step, gx, bx, gy, by, ClampedCellSampler2{cs, xmax, ymax}, seg, last,
-                                       end_val, last_step, holds_last, whole);
-        } else {
-            pixel = march_ray<SEG>(a, am, step, gx, bx, gy, by, BorderSampler<T>{vol + (size_t)b * X * Y, X, Y},
-                                   seg, last, end_val, last_step, holds_last, whole);
-        }
+    float sum[NS], last[NS], end_val[NS], last_step = 0.0f;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) sum[s] = last[s] = end_val[s] = 0.0f;
+    bool holds_last = false;
+    const bool hit = live && ray.step > 0.0f && amin < amax;
+    // sample positions in index space: idx = (src + a r - o) / s; the major
+    // axis is the one the view's rays run mostly along (fan: the central ray)
+    const bool along_x = fabsf(ray_in.x) > fabsf(ray_in.y);
+    const float bx = (float)((srcx - ox) / sx), by = (float)((srcy - oy) / sy);
+    const float gx = dx * (1.0f / sx), gy = dy * (1.0f / sy);
+    ray.bm = along_x ? bx : by, ray.bn = along_x ? by : bx;
+    ray.gm = along_x ? gx : gy, ray.gn = along_x ? gy : gx;
+    ray.a = (float)amin;
+    ray.am = (float)amax;
+    const int M = along_x ? X : Y, N = along_x ? Y : X;
+    // the last slices of a batch that NS does not divide: the thread's
+    // slices are the batch's last NS
+    const int b0 = NS == 1 ? b : min(b, batch - NS);
+    if (cells_x) {
+        const size_t slice = (size_t)(X + 3) * (Y + 3);
+        const float4 *cells = (along_x ? cells_y : cells_x) + b0 * slice;
+        const unsigned pitch = N + 3;
+        // every position of the march lies between its two end points (half a
+        // cell of slack for the rounding of the positions)
+        const float m0 = ray.m(ray.a), n0 = ray.n(ray.a), m1 = ray.m(ray.am), n1 = ray.n(ray.am);
+        const float mmax = (float)M + 0.5f, nmax = (float)N + 0.5f;
+        const bool inside = hit && m0 >= -1.5f && m1 >= -1.5f && m0 <= mmax && m1 <= mmax && n0 >= -1.5f &&
+                            n1 >= -1.5f && n0 <= nmax && n1 <= nmax && max(X, Y) < (1 << 20);
+        const unsigned mask = __ballot_sync(0xffffffffu, inside);
+        if (inside)
+            march_ray<SEG, NS>(ray, CellTaps<false>{cells, slice, pitch, M, N}, mask, seg, M, sum, last, end_val,
+                               last_step, holds_last);
+        else if (hit)
+            march_ray<SEG, NS>(ray, CellTaps<true>{cells, slice, pitch, M, N}, 0u, seg, M, sum, last, end_val, last_step,
+                               holds_last);
+    } else if (hit) {
+        const size_t slice = (size_t)X * Y;
+        march_ray<SEG, NS>(ray, BorderTaps<T>{vol + b0 * slice, slice, along_x ? 1 : X, along_x ? X : 1, M, N}, 0u, seg, M,
+                           sum, last, end_val, last_step, holds_last);
     }
     if (SEG > 1) {
-        // range sums in order, then march2d's scaling and end correction
         __shared__ float s_sum[SEG][RAYS];
         __shared__ float s_last[RAYS], s_end[RAYS], s_step[RAYS];
-        __shared__ int s_whole[RAYS];
-        s_sum[seg][lane] = pixel;
-        if (holds_last) s_last[lane] = last, s_end[lane] = end_val, s_step[lane] = last_step;
-        if (seg == 0) s_whole[lane] = whole;
+        s_sum[seg][lane] = sum[0];
+        if (holds_last) s_last[lane] = last[0], s_end[lane] = end_val[0], s_step[lane] = last_step;
         __syncthreads();
-        if (seg != 0 || !live) return;
-        if (!s_whole[lane]) {
-            pixel = s_sum[0][lane];
+        if (seg != 0) return;
 #pragma unroll
-            for (int r = 1; r < SEG; ++r) pixel += s_sum[r][lane];
-            pixel *= step;
-            if (pixel > 0.0f) {  // a sample exists: some range held the last one
-                pixel -= 0.5f * step * s_last[lane];
-                pixel += 0.5f * s_step[lane] * s_last[lane];
-                pixel += 0.5f * s_step[lane] * s_end[lane];
-            }
-        }
+        for (int r = 1; r < SEG; ++r) sum[0] += s_sum[r][lane];
+        if (sum[0] != 0.0f) last[0] = s_last[lane], end_val[0] = s_end[lane], last_step = s_step[lane];
     }
-    pixel *= sqrtf((dx * sx) * (dx * sx) + (dy * sy) * (dy * sy));  // :141
-    store_from_float(sino + ((size_t)b * n_proj + p) * W + u, pixel);
+    if (!live) return;
+    const float scale = sqrtf((dx * sx) * (dx * sx) + (dy * sy) * (dy * sy));  // :141
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        float pixel = sum[s] * ray.step;
+        if (pixel > 0.0f) {  // :88-100
+            pixel -= 0.5f * ray.step * last[s];
+            pixel += 0.5f * last_step * last[s];
+            pixel += 0.5f * last_step * end_val[s];
+        }
+        const int bs = NS == 1 ? b : min(b, batch - NS) + s;
+        store_from_float(sino + ((size_t)bs * n_proj + p) * W + u, pixel * scale);
+    }
 }
 
 // Linear interpolation of a sinogram row at floor x0 with weight t, taps
@@ -700,13 +707,13 @@ __global__ void __launch_bounds__(256) pad_cells2d_kernel(const T *__restrict__ 
         {  // x-fastest: thread x along xc
             const int xc = xc0 + threadIdx.x, yc = yc0 + r;
             if (xc < Xc && yc < Yc)
-                cells_x[slice + (size_t)yc * Xc + xc] = Cell2::make(
-                    tile[r][threadIdx.x], tile[r][threadIdx.x + 1], tile[r + 1][threadIdx.x], tile[r + 1][threadIdx.x + 1]);
+                cells_x[slice + (size_t)yc * Xc + xc] = make_float4(
+                    tile[r][threadIdx.x], tile[r + 1][threadIdx.x], tile[r][threadIdx.x + 1], tile[r + 1][threadIdx.x + 1]);
         }
         {  // y-fastest: thread x along yc
             const int yc = yc0 + threadIdx.x, xc = xc0 + r;
             if (xc < Xc && yc < Yc)
-                cells_y[slice + (size_t)xc * Yc + yc] = Cell2::make(
+                cells_y[slice + (size_t)xc * Yc + yc] = make_float4(
                     tile[threadIdx.x][r], tile[threadIdx.x][r + 1], tile[threadIdx.x + 1][r], tile[threadIdx.x + 1][r + 1]);
         }
     }
@@ -726,19 +733,32 @@ cudaError_t fp_typed(const void *volume, void *sinogram, bool fan, const Dims2D 
         pad_cells2d_kernel<Tin><<<tgrid, dim3(32, 8), 0, stream>>>((const Tin *)volume, cells_x, cells_y, d.vol_x,
                                                                   d.vol_y);
     }
-    // segments per ray for launches of few rays (see SEG2D)
-    const bool segs = (long long)d.batch * d.n_proj * d.det_w <= SEG2D_MAX_RAYS;
+    // segments per ray for launches of few rays (see SEG2D), else up to four
+    // slices of one geometry per thread (the walk costs a visit about 33
+    // instructions, a slice 9 more: 64 fan slices of 512^2, FP16, 41.4 -> 21.7 ms
+    // by cell visits and four slices per thread, 13.2 ms with aligned columns,
+    // 12.0 ms on packed instructions; eight slices per thread 12.2 ms)
+    const bool share = d.geom_batch == 1 && d.batch >= 2;
+    const bool segs = (long long)d.batch * d.n_proj * d.det_w <= (share ? SEG2D_MAX_RAYS_SHARED : SEG2D_MAX_RAYS);
+    const int ns = segs || !share ? 1 : (d.batch >= 4 ? 4 : 2);
     const int rays = segs ? FP2_BLOCK / SEG2D : FP2_BLOCK;
-    const dim3 grid((d.det_w + rays - 1) / rays, d.n_proj, d.batch);
+    const dim3 grid((d.det_w + rays - 1) / rays, d.n_proj, (d.batch + ns - 1) / ns);
     auto launch = [&](auto kernel) {
         kernel<<<grid, FP2_BLOCK, 0, stream>>>((const Tin *)volume, cells_x, cells_y, (Tout *)sinogram, g, d.vol_x,
-                                               d.vol_y, d.det_w, d.n_proj, d.geom_batch);
+                                               d.vol_y, d.det_w, d.n_proj, d.batch, d.geom_batch);
     };
-    if (fan)
-        segs ? launch(projection2d_kernel<Tin, Tout, true, SEG2D>) : launch(projection2d_kernel<Tin, Tout, true, 1>);
-    else
-        segs ? launch(projection2d_kernel<Tin, Tout, false, SEG2D>)
-             : launch(projection2d_kernel<Tin, Tout, false, 1>);
+    auto launch_beam = [&](auto fan_c) {
+        constexpr bool FAN = decltype(fan_c)::value;
+        if (segs)
+            launch(projection2d_kernel<Tin, Tout, FAN, SEG2D, 1>);
+        else if (ns == 4)
+            launch(projection2d_kernel<Tin, Tout, FAN, 1, 4>);
+        else if (ns == 2)
+            launch(projection2d_kernel<Tin, Tout, FAN, 1, 2>);
+        else
+            launch(projection2d_kernel<Tin, Tout, FAN, 1, 1>);
+    };
+    fan ? launch_beam(std::true_type{}) : launch_beam(std::false_type{});
     return cudaGetLastError();
 }
 

@@ -1,0 +1,83 @@
+"""GPU parity of the kernels' size- and geometry-dependent paths against the
+FP64 oracle, at the sizes where each path begins, ends or wraps.
+
+Tolerances (relative L2) are those of test_ops_gpu.py: FP32 arithmetic on the
+same (storage-rounded) input, 2e-5 for ray marches, 1e-5 for backprojections.
+"""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import pyronn_layers as pl
+from pyronn_layers import _capi, geometry
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def t(a, dev, dtype=torch.float32):
+    return torch.as_tensor(np.asarray(a)).to(device=dev, dtype=dtype)
+
+
+def noise(seed, shape):
+    return np.random.Generator(np.random.PCG64(seed)).uniform(0.2, 1.0, shape).astype(np.float32)
+
+
+# ------------------------------------------------------------- 2D forward
+
+
+@pytest.mark.parametrize("fan", [False, True])
+@pytest.mark.parametrize("batch,views,width", [
+    (1, 9, 40),      # ray segments (one band of columns per thread)
+    (1, 97, 3100),   # one thread per ray, one slice (above the segments' limit)
+    (2, 97, 780),    # two slices per thread
+    (3, 83, 610),    # two slices per thread, the last pair overlapping
+    (4, 83, 460),    # four slices per thread
+    (5, 61, 500),    # four per thread, the last group overlapping
+])
+def test_2d_forward_walks(cuda, batch, views, width, fan):
+    """Every walk of the 2D forward (segments; one, two and four slices per
+    thread) against the oracle, and without the workspace the same bits."""
+    shape, sp, ds = (23, 37), (0.8, 1.0), 60.0 / width
+    if fan:
+        geo = geometry.FanBeam2D(shape, sp, width, ds, views, 60.0, 90.0)
+        fwd, ofwd, name = pl.fan_projection2d, oracle.fan_projection2d, "pyronn_fan_projection2d"
+    else:
+        geo = geometry.ParallelBeam2D(shape, sp, width, ds, views)
+        fwd, ofwd, name = pl.parallel_projection2d, oracle.parallel_projection2d, "pyronn_parallel_projection2d"
+    img = noise(batch, (batch,) + shape)
+    out = fwd(t(img, cuda), geo.detector_shape, *geo.args())
+    ref = ofwd(img, geo.detector_shape, *geo.args())
+    assert rel_l2(out.cpu().numpy(), ref) < 2e-5
+    gp = pl.ops.Geometry2D(batch, cuda, *geo.args()[:4], geo.args()[-1], views, *(geo.args()[4:6] if fan else ()))
+    plain = torch.empty_like(out)
+    x = t(img, cuda)
+    _capi.call(name, x.data_ptr(), plain.data_ptr(), 0, 0, batch, *shape, views, width, *gp.pointers(), gp.g, 0, 0,
+               torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(plain, out)
+
+
+@pytest.mark.parametrize("spacing", [(1.0, 1.0), (0.8, 1.3), (0.05, 0.05), (5.0 * 2.0 ** -3 * (1 + 2.0 ** -12),) * 2])
+@pytest.mark.parametrize("length", [1.0, 0.37, 40.0])
+def test_2d_forward_alpha_sequences(cuda, spacing, length):
+    """Ray vectors of any length (steps of a fraction of a cell up to several
+    cells), steps whose float sums are ties, and rays whose alphas cross
+    binades: the samples sit where the one-at-a-time float march puts them."""
+    shape, views, width = (33, 29), 24, 51
+    geo = geometry.ParallelBeam2D(shape, spacing, width, 40.0 * max(spacing) / width, views)
+    args = geo.args()[:4] + (geo.ray_vectors * np.float32(length),)
+    img = noise(5, (1,) + shape)
+    out = pl.parallel_projection2d(t(img, cuda), (views, width), *args)
+    ref = oracle.parallel_projection2d(img, (views, width), *args)
+    assert rel_l2(out.cpu().numpy(), ref) < 2e-5
+
+
+def test_2d_forward_source_inside(cuda):
+    """A fan source inside the slice: the march starts at negative alphas."""
+    geo = geometry.FanBeam2D((40, 40), (1.0, 1.0), 64, 1.0, 16, 9.0, 40.0)
+    img = noise(6, (2, 40, 40))
+    out = pl.fan_projection2d(t(img, cuda), geo.detector_shape, *geo.args())
+    ref = oracle.fan_projection2d(img, geo.detector_shape, *geo.args())
+    assert rel_l2(out.cpu().numpy(), ref) < 2e-5
