@@ -81,3 +81,47 @@ def test_2d_forward_source_inside(cuda):
     out = pl.fan_projection2d(t(img, cuda), geo.detector_shape, *geo.args())
     ref = oracle.fan_projection2d(img, geo.detector_shape, *geo.args())
     assert rel_l2(out.cpu().numpy(), ref) < 2e-5
+
+
+# ---------------------------------------------------------- 2D backprojection
+
+
+@pytest.mark.parametrize("fan", [False, True])
+@pytest.mark.parametrize("batch,shape,views,width,dtype", [
+    (1, (33, 65), 70, 90, torch.float32),       # one slice, view groups
+    (2, (31, 33), 257, 60, torch.bfloat16),     # two slices per thread; two view chunks
+    (3, (40, 37), 33, 91, torch.float32),       # two per thread, the last pair overlapping
+    (5, (40, 37), 33, 30, torch.float16),       # four per thread, overlapping; pixels off the detector
+])
+def test_2d_backprojection_walks(cuda, batch, shape, views, width, dtype, fan):
+    """The splits of the 2D backprojection (view groups; one, two and four
+    slices per thread; blocks wholly inside the detector rows and blocks that
+    need tap flags) against the oracle."""
+    if fan:
+        geo = geometry.FanBeam2D(shape, (0.8, 1.0), width, 1.1, views, 900.0, 1300.0)
+        bwd, obwd = pl.fan_backprojection2d, oracle.fan_backprojection2d
+    else:
+        geo = geometry.ParallelBeam2D(shape, (0.8, 1.0), width, 0.9, views)
+        bwd, obwd = pl.parallel_backprojection2d, oracle.parallel_backprojection2d
+    p = t(noise(batch, (batch,) + geo.detector_shape), cuda, dtype)
+    out = bwd(p, geo.volume_shape, *geo.args(), out_dtype=torch.float32)
+    ref = obwd(p.float().cpu().numpy(), geo.volume_shape, *geo.args())
+    assert rel_l2(out.cpu().numpy(), ref) < 1e-5
+
+
+@pytest.mark.parametrize("fan", [False, True])
+@pytest.mark.parametrize("batch,shape,dtype", [(6, (900, 800), torch.float32), (9, (960, 940), torch.float16)])
+def test_2d_backprojection_shared_slices(cuda, batch, shape, dtype, fan):
+    """Launches without view groups: four and eight slices per thread (the last
+    group overlapping) give each slice the bits of a call of its own."""
+    if fan:
+        geo = geometry.FanBeam2D(shape, (0.8, 1.0), 2000, 1.1, 3, 900.0, 1300.0)
+        bwd = pl.fan_backprojection2d
+    else:
+        geo = geometry.ParallelBeam2D(shape, (0.8, 1.0), 2000, 0.9, 3)
+        bwd = pl.parallel_backprojection2d
+    p = t(noise(batch, (batch,) + geo.detector_shape), cuda, dtype)
+    out = bwd(p, geo.volume_shape, *geo.args(), out_dtype=torch.float32)
+    for b in range(batch):
+        one = bwd(p[b:b + 1], geo.volume_shape, *geo.args(), out_dtype=torch.float32)
+        assert torch.equal(one[0], out[b])
