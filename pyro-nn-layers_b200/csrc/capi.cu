@@ -311,7 +311,7 @@ size_t pyronn_cone_projection3d_workspace_size(int batch, int vol_z, int vol_y, 
         return 0;
     size_t n = WS_HEADER + align_up((size_t)geom_batch * n_proj * sizeof(ConeFpView), 256);
     const Dims3D d{batch, vol_z, vol_y, vol_x, n_proj, det_h, det_w, geom_batch};
-    if (!hardware_interp && cone_fp_padded_supported(d))
+    if (!hardware_interp && cone_fp_padded_supported(d, in_dtype))
         n += align_up(cone_fp_padded_scratch_bytes(vol_z, vol_y, vol_x, in_dtype), 256);
     return n;
 }
@@ -370,7 +370,7 @@ int pyronn_cone_projection3d(const void *volume, void *sinogram, int in_dtype, i
                                vol_z, views, s);
     if (e != cudaSuccess) return cuda_fail(e, "cone_projection3d: geometry preparation");
     if (!hardware_interp) {
-        if (cone_fp_padded_supported(d)) {
+        if (cone_fp_padded_supported(d, in_dtype)) {
             void *scratch = (char *)workspace + WS_HEADER +
                             align_up((size_t)geom_batch * n_proj * sizeof(ConeFpView), 256);
             e = launch_cone_fp_padded(volume, sinogram, in_dtype, out_dtype, d, views, step_size, volume_spacing,

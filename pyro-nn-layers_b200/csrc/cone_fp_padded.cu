@@ -49,9 +49,15 @@ __global__ void classify_views_kernel(const ConeFpView *__restrict__ views, int 
     atomicOr(&flags[view_is_z_mode(views[t]) ? FLAG_NEED_Z : FLAG_NEED_XY], 1u);
 }
 
-// The eight taps of a trilinear cell, as (x0, x1) pairs in the order
-// (y0 z0), (y0 z1), (y1 z0), (y1 z1): two float4 for FP32, four 32-bit words
-// of two 16-bit values for BF16 / FP16 (x0 in the low half).  The 16-bit
+// A cell of FP32 storage holds the four taps of its z0 plane; the z1 plane is
+// the next cell along z, so a sample is two adjacent 16-byte loads and the
+// lanes' loads (consecutive z) overlap.  With all eight taps in a cell (32
+// bytes) a warp's two loads touched twice the lines: with four taps and the
+// packed lerps the FP32 forward takes 171.3 -> 119.5 ms at 512^3 (360 views of
+// 1024 x 768), 2.29 -> 1.79 ms at 128^3 (180 views of 256^2; 73 % issue active, the
+// L1 61 % busy), the same bits.  A cell of 16-bit storage holds
+// the eight taps as (x0, x1) pairs in the order (y0 z0), (y0 z1), (y1 z0),
+// (y1 z1): four 32-bit words of two values (x0 in the low half).  The 16-bit
 // cells hold the z0 taps and, in place of the z1 taps, the half-differences
 // (z1 - z0) / 2 rounded to the storage type (the halving keeps every FP16
 // difference finite).  Their z lerp z0 + (2t) ((z1 - z0) / 2) takes 16-bit
@@ -66,10 +72,6 @@ __global__ void classify_views_kernel(const ConeFpView *__restrict__ views, int 
 // oracle stays the storage rounding's (FP16 2.65e-4), measured at 96.8 ms
 // (widened taps, FP32 lerps) -> 90.0 ms (mixed z lerps) -> 83.0 ms (packed)
 // -> 75.4 ms (other changes) -> 73.0 ms (y-difference cells).
-struct alignas(16) CellF32 {
-    float4 y0, y1;  // (x0 z0, x1 z0, x0 z1, x1 z1) at y0, then at y1
-};
-
 // z0 + t2 * hd for the z0 tap in word `a` and the half-difference in word
 // `d` (the half selected by HI) and t2 = 2t in the storage type
 template <bool BF16, bool HI>
@@ -100,33 +102,24 @@ template <typename T>
 struct Cell;
 template <>
 struct Cell<float> {
-    using type = CellF32;
-    __device__ static void load(const CellF32 *c, float (&v)[8])
+    using type = float4;  // (x0 y0, x1 y0, x0 y1, x1 y1) at one z
+    static constexpr int PLANES = 3;  // z entries beyond the volume: floors [-1, Z], and the next
+    // z lerps of the (x0, x1) pairs at y0 and y1, y lerp of the pair, x lerp:
+    // the reference's form throughout (lerp_ref), pairs on the packed FP32
+    // instructions
+    __device__ static float2 lerp2(float2 a, float2 b, float t)
     {
-        const float4 a = __ldg(&c->y0), b = __ldg(&c->y1);
-        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        return __ffma2_rn(b, make_float2(t, t), __ffma2_rn(a, make_float2(-t, -t), a));
     }
-    // the four z lerps of a cell: z[0] = (x0 y0), z[1] = (x1 y0), z[2] = (x0 y1), z[3] = (x1 y1)
-    __device__ static void zlerp(const CellF32 *c, float t, float (&z)[4])
+    __device__ static float trilinear(const float4 *c, float tz, float ty, float tx)
     {
-        float v[8];
-        load(c, v);
-        z[0] = lerp_ref(v[0], v[2], t), z[1] = lerp_ref(v[1], v[3], t);
-        z[2] = lerp_ref(v[4], v[6], t), z[3] = lerp_ref(v[5], v[7], t);
+        const float4 a = __ldg(c), b = __ldg(c + 1);
+        const float2 y0 = lerp2(make_float2(a.x, a.y), make_float2(b.x, b.y), tz);
+        const float2 y1 = lerp2(make_float2(a.z, a.w), make_float2(b.z, b.w), tz);
+        const float2 v = lerp2(y0, y1, ty);
+        return lerp_ref(v.x, v.y, tx);
     }
-    __device__ static float trilinear(const CellF32 *c, float tz, float ty, float tx)
-    {
-        float zl[4];
-        zlerp(c, tz, zl);
-        return lerp_ref(lerp_ref(zl[0], zl[2], ty), lerp_ref(zl[1], zl[3], ty), tx);
-    }
-    __device__ static CellF32 make(const float (&v)[8])
-    {
-        CellF32 c;
-        c.y0 = make_float4(v[0], v[1], v[2], v[3]);
-        c.y1 = make_float4(v[4], v[5], v[6], v[7]);
-        return c;
-    }
+    __device__ static float4 make(const float (&v)[8]) { return make_float4(v[0], v[1], v[4], v[5]); }
 };
 // the 16-bit cells: words (z0 taps at y0, half-differences at y0, z0 taps
 // at y1, half-differences at y1) -- or, for the packed lerps, the last two
@@ -135,6 +128,7 @@ template <typename T16>
 struct Cell16 {
     static constexpr bool BF16 = std::is_same<T16, __nv_bfloat16>::value;
     using type = uint4;
+    static constexpr int PLANES = 2;  // z entries beyond the volume: floors [-1, Z]
     __device__ static void zlerp(const uint4 *c, float t, float (&z)[4])
     {
         const uint4 w = __ldg(c);
@@ -251,8 +245,8 @@ struct Wide16<__nv_bfloat16> {
 };
 
 // z-fastest cell copy: element [xc][yc][zc], xc in [0, X+1] (pitch s_x >=
-// (Y+2) (Z+2), from cell_x_pitch), yc in [0, Y+1], zc in [0, Z+1], holds the
-// cell whose low corner is voxel (xc-1, yc-1, zc-1)
+// (Y+2) Zc, from cell_x_pitch), yc in [0, Y+1], zc in [0, Zc), Zc = Z + PLANES,
+// holds the cell whose low corner is voxel (xc-1, yc-1, zc-1)
 // (V zero outside the volume), i.e. the taps of every floor in [-1, N].
 // A block reads a 33 (x) x 33 (z) x (CELL_PLANES + 1) (y) tile along x --
 // each plane once for its CELL_PLANES cell planes -- and writes 32 (z) x 32
@@ -286,7 +280,7 @@ __global__ void __launch_bounds__(PAD_TILE *8) pad_cells_kernel(const T *__restr
     __shared__ T tile[CELL_PLANES + 1][PAD_TILE + 1][PAD_TILE + 2];
     // 16-bit inputs within range take the packed lerps' y-difference cells
     const bool ydiff = sizeof(T) == 2 && !flags[FLAG_WIDE];
-    const int Yc = Y + 2, Zc = Z + 2;
+    const int Yc = Y + 2, Zc = Z + Cell<T>::PLANES;
     const int xc0 = blockIdx.x * PAD_TILE, yc0 = blockIdx.y * CELL_PLANES, zc0 = blockIdx.z * PAD_TILE;
     for (int rr = threadIdx.y; rr < (CELL_PLANES + 1) * (PAD_TILE + 1); rr += 8) {
         const int dy = rr / (PAD_TILE + 1), r = rr % (PAD_TILE + 1);
@@ -406,18 +400,6 @@ struct ClampedSampler {
     }
 };
 
-// true when every point of the FP32 march lies in [-0.5, N + 0.5]: its end
-// points do (the segment between is convex) -- checked once per ray
-__device__ __forceinline__ bool march_inside(const ConeRay &r, int X, int Y, int Z)
-{
-    if (!r.hit) return true;
-    const float x0 = fmaf(r.a, r.dx, r.ox), y0 = fmaf(r.a, r.dy, r.oy), z0 = fmaf(r.a, r.dz, r.oz);
-    const float x1 = fmaf(r.am, r.dx, r.ox), y1 = fmaf(r.am, r.dy, r.oy), z1 = fmaf(r.am, r.dz, r.oz);
-    const float lo = -0.5f;
-    return fminf(x0, x1) >= lo && fminf(y0, y1) >= lo && fminf(z0, z1) >= lo && fmaxf(x0, x1) <= X + 0.5f &&
-           fmaxf(y0, y1) <= Y + 0.5f && fmaxf(z0, z1) <= Z + 0.5f;
-}
-
 // floor and fraction of z2 / 2 from z2 = 2 z (exact: scaling by two commutes
 // with every rounding here): bits = floor(z) + FLOOR_BIAS_2Z, f = 2 (z - floor(z))
 constexpr int FLOOR_BIAS_2Z = 0x4BC00000;  // bit pattern of 1.5 * 2^24
@@ -489,10 +471,9 @@ __device__ __forceinline__ float march_cells(const ConeRay &ray, float step, boo
                                              const typename Cell<T>::type *cells, int Z, int s_x, float xmax,
                                              float ymax, float zmax)
 {
-    const CellSampler<T, PACKED> s(cells, Z + 2, s_x);
+    const CellSampler<T, PACKED> s(cells, Z + Cell<T>::PLANES, s_x);
     const int n = inside ? exact_sample_count(ray, step) : -1;
-    // samples per iteration: four for the 32-byte FP32 cells (whose loads
-    // need twice the registers), seven for FP16 and six for BF16 cells
+    // samples per iteration: four for FP32 cells (two loads a sample), seven for FP16 and six for BF16 cells
     // (measured on the 512^3 forward, the best of a sweep whose times follow
     // the compiler's schedule more than the count: FP16 4 / 5 / 6 / 7 / 8 per
     // iteration 82.3 / 80.3 / 79.0 / 77.2 / 77.4 ms; BF16 5 / 6 / 7 / 8 / 10:
@@ -587,15 +568,21 @@ size_t section_bytes(size_t n)
     return (n + 255) / 256 * 256;
 }
 
-// x pitch (in cells) of the cell copy: the least s_x >= (Y+2) (Z+2) for which
+// z entries of a column of the cell copy beyond the volume's
+int cell_planes(size_t elem)
+{
+    return elem == 4 ? Cell<float>::PLANES : Cell<__half>::PLANES;
+}
+
+// x pitch (in cells) of the cell copy: the least s_x >= (Y+2) Zc for which
 // the sampler's biased index, cell_index_bias + index, stays in [0, 2^32) for
 // every index of the copy relative to floor (0, 0, 0) -- from -(s_x + s_y + 1)
 // up to below (X+2) s_x -- under both z floors; 0 when none is found.  The
 // bias moves by FLOOR_BIAS (mod 2^32) per unit of s_x, which steps through all
 // 1024 multiples of 2^22, so a few units of padding suffice.
-long long cell_x_pitch(int vol_x, int vol_y, int vol_z)
+long long cell_x_pitch(int vol_x, int vol_y, int vol_z, size_t elem)
 {
-    const unsigned long long Xc = vol_x + 2, Yc = vol_y + 2, Zc = vol_z + 2;
+    const unsigned long long Xc = vol_x + 2, Yc = vol_y + 2, Zc = vol_z + cell_planes(elem);
     for (unsigned long long sx = Yc * Zc; sx < Yc * Zc + 2048 && Xc * sx < (1ULL << 31); ++sx) {
         bool ok = true;
         for (const bool z2 : {false, true}) {
@@ -613,8 +600,8 @@ cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, co
 {
     using CellT = typename Cell<Tin>::type;
     const size_t Xp = d.vol_x + 3, Yp = d.vol_y + 3, Zp = d.vol_z + 3;
-    const size_t Xc = d.vol_x + 2, Yc = d.vol_y + 2, Zc = d.vol_z + 2;
-    const long long cell_sx = cell_x_pitch(d.vol_x, d.vol_y, d.vol_z);
+    const size_t Xc = d.vol_x + 2, Yc = d.vol_y + 2, Zc = d.vol_z + Cell<Tin>::PLANES;
+    const long long cell_sx = cell_x_pitch(d.vol_x, d.vol_y, d.vol_z, sizeof(Tin));
     if (cell_sx <= 0) return cudaErrorInvalidValue;
     char *base = (char *)scratch;
     Tin *xfast = (Tin *)base;
@@ -655,15 +642,19 @@ size_t cone_fp_padded_scratch_bytes(int vol_z, int vol_y, int vol_x, int in_dtyp
 {
     const size_t e = dtype_size(in_dtype);
     const size_t padded = (size_t)(vol_x + 3) * (vol_y + 3) * (vol_z + 3);
-    const size_t cells = (size_t)(vol_x + 2) * (size_t)cell_x_pitch(vol_x, vol_y, vol_z);
-    return 2 * section_bytes(padded * e) + section_bytes(cells * 8 * e);
+    const size_t cells = (size_t)(vol_x + 2) * (size_t)cell_x_pitch(vol_x, vol_y, vol_z, e);
+    // (the query's answer is eight taps per cell for every type; FP32 cells,
+    // of four taps, use about half of it)
+    const size_t taps8 = (size_t)(vol_x + 2) * (vol_y + 2) * (vol_z + 2) * 8 * e;
+    return 2 * section_bytes(padded * e) + section_bytes(std::max(cells * 16, taps8));
 }
 
-bool cone_fp_padded_supported(const Dims3D &d)
+bool cone_fp_padded_supported(const Dims3D &d, int in_dtype)
 {
     const long long padded = (long long)(d.vol_x + 3) * (d.vol_y + 3) * (d.vol_z + 3);
     return padded < (1LL << 31) - (1LL << 20) && ray_blocks_fit(d.det_w, d.det_h, d.n_proj) &&
-           d.vol_z + 3 <= 65535 && d.vol_y + 3 <= 65535 && cell_x_pitch(d.vol_x, d.vol_y, d.vol_z) > 0;
+           d.vol_z + 3 <= 65535 && d.vol_y + 3 <= 65535 &&
+           cell_x_pitch(d.vol_x, d.vol_y, d.vol_z, dtype_size(in_dtype)) > 0;
 }
 
 cudaError_t launch_cone_fp_padded(const void *volume, void *sinogram, int in_dtype, int out_dtype, const Dims3D &d,

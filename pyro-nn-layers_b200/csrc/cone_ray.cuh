@@ -83,6 +83,18 @@ __device__ __forceinline__ ConeRay cone_ray_setup(const ConeFpView &view, int u,
     return ray;
 }
 
+// true when every point of the FP32 march lies in [-0.5, N + 0.5]: its end
+// points do (the segment between is convex) -- checked once per ray
+__device__ __forceinline__ bool march_inside(const ConeRay &r, int X, int Y, int Z)
+{
+    if (!r.hit) return true;
+    const float x0 = fmaf(r.a, r.dx, r.ox), y0 = fmaf(r.a, r.dy, r.oy), z0 = fmaf(r.a, r.dz, r.oz);
+    const float x1 = fmaf(r.am, r.dx, r.ox), y1 = fmaf(r.am, r.dy, r.oy), z1 = fmaf(r.am, r.dz, r.oz);
+    const float lo = -0.5f;
+    return fminf(x0, x1) >= lo && fminf(y0, y1) >= lo && fminf(z0, z1) >= lo && fmaxf(x0, x1) <= X + 0.5f &&
+           fmaxf(y0, y1) <= Y + 0.5f && fmaxf(z0, z1) <= Z + 0.5f;
+}
+
 // Block order of the ray-driven forward kernels.  The grid is one
 // dimension; each 32 x 32 tile of detector rays of a view is four blocks of
 // 256 threads (sub = 0..3).  Views go in chunks of VIEW_CHUNK; inside a chunk

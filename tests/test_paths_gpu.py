@@ -125,3 +125,17 @@ def test_2d_backprojection_shared_slices(cuda, batch, shape, dtype, fan):
     for b in range(batch):
         one = bwd(p[b:b + 1], geo.volume_shape, *geo.args(), out_dtype=torch.float32)
         assert torch.equal(one[0], out[b])
+
+
+# -------------------------------------------------------------- cone forward
+
+
+def test_cone_forward_fp32_cell_pitch(cuda):
+    """A volume (60 x 8 x 60, z y x) whose FP32 cell copy (three z entries
+    beyond the volume) needs a padded x pitch for its biased index not to
+    wrap, with rays through its upper z face."""
+    geo = geometry.ConeBeam3D((60, 8, 60), (1.0, 1.0, 1.0), (64, 40), (2.5, 2.0), 6, 90.0, 170.0, step_size=0.5)
+    vol = noise(12, (2,) + geo.volume_shape)
+    out = pl.cone_projection3d(t(vol, cuda), geo.detector_shape, *geo.args())
+    ref = oracle.cone_projection3d(vol, geo.detector_shape, *geo.args())
+    assert rel_l2(out.cpu().numpy(), ref) < 2e-5
