@@ -230,6 +230,13 @@ PYRONN_API int pyronn_cone_backprojection3d(const void *sinogram, void *volume, 
  *   vol_y, vol_x] FP32 (overwritten); projection_multiplier is not applied.
  * ------------------------------------------------------------------------- */
 PYRONN_API size_t pyronn_cone_backprojection3d_matched_workspace_size(int geom_batch, int n_proj);
+/* The per-view part above plus cell accumulators of one volume (16 bytes per
+ * cell, about four times the FP32 volume): with a workspace of this size the
+ * rays scatter 16-byte vectors into the accumulators, several times faster than
+ * single atomics into the volume; a smaller one is accepted, as above. */
+PYRONN_API size_t pyronn_cone_backprojection3d_matched_cells_workspace_size(int geom_batch, int n_proj, int det_h,
+                                                                            int det_w, int vol_z, int vol_y,
+                                                                            int vol_x);
 
 PYRONN_API int pyronn_cone_backprojection3d_matched(const void *sinogram, float *volume, int in_dtype, int batch,
                                                     int n_proj, int det_h, int det_w, int vol_z, int vol_y,

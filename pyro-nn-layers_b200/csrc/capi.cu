@@ -461,6 +461,15 @@ size_t pyronn_cone_backprojection3d_matched_workspace_size(int geom_batch, int n
     return WS_HEADER + align_up((size_t)geom_batch * n_proj * sizeof(ConeFpView), 256);
 }
 
+size_t pyronn_cone_backprojection3d_matched_cells_workspace_size(int geom_batch, int n_proj, int det_h, int det_w,
+                                                                 int vol_z, int vol_y, int vol_x)
+{
+    const size_t views = pyronn_cone_backprojection3d_matched_workspace_size(geom_batch, n_proj);
+    if (views == 0 || det_h <= 0 || det_w <= 0 || vol_z <= 0 || vol_y <= 0 || vol_x <= 0) return 0;
+    if (!cone_ray_grid_fits(det_w, det_h, n_proj)) return views;
+    return views + align_up(cone_scatter_cells_bytes(vol_z, vol_y, vol_x), 256);
+}
+
 int pyronn_cone_backprojection3d_matched(const void *sinogram, float *volume, int in_dtype, int batch, int n_proj,
                                          int det_h, int det_w, int vol_z, int vol_y, int vol_x,
                                          const float *volume_origin, const float *volume_spacing,
@@ -488,7 +497,14 @@ int pyronn_cone_backprojection3d_matched(const void *sinogram, float *volume, in
     if (e == cudaSuccess)
         e = launch_cone_fp_prepare(projection_matrices, volume_spacing, volume_origin, geom_batch, n_proj, vol_x,
                                    vol_y, vol_z, views, s);
-    if (e == cudaSuccess) e = launch_cone_scatter(sinogram, volume, in_dtype, d, views, step_size, volume_spacing, s);
+    // cell accumulators where the workspace holds them
+    const size_t cells = pyronn_cone_backprojection3d_matched_cells_workspace_size(geom_batch, n_proj, det_h, det_w,
+                                                                                   vol_z, vol_y, vol_x);
+    if (e == cudaSuccess && cells > need && workspace_bytes >= cells)
+        e = launch_cone_scatter_cells(sinogram, volume, in_dtype, d, views, step_size, volume_spacing,
+                                      (char *)workspace + need, s);
+    else if (e == cudaSuccess)
+        e = launch_cone_scatter(sinogram, volume, in_dtype, d, views, step_size, volume_spacing, s);
     if (e != cudaSuccess) return cuda_fail(e, name);
     return ok();
 }

@@ -9,6 +9,14 @@
 // weight into the eight taps with FP32 atomics: the result is A^T y for the
 // linear forward operator, which equals the reference forward projector on
 // every ray whose line integral is > 0 (e.g. any non-negative volume).
+//
+// Given a workspace for them, the rays scatter into CELL accumulators, the
+// transpose of the forward's FP32 cell copy: element (x, y, z), z fastest, sums
+// what falls on the taps V(x + {0,1}, y + {0,1}) at z, so a sample is two
+// adjacent 16-byte vector additions instead of eight scalar atomics to eight
+// rows; a second kernel adds each voxel's four cell entries.  Views whose
+// detector v axis runs along z lay warps along v, like the forward: a warp's
+// additions fall on consecutive cells.  What bounds it: the L2's additions.
 #include "common.cuh"
 #include "cone_ray.cuh"
 #include "internal.h"
@@ -71,7 +79,175 @@ __global__ void __launch_bounds__(MB_X *MB_Y)
     });
 }
 
+// z entries of a column of cell accumulators beyond the volume's: floors
+// [-1, Z] and the next
+constexpr int ACC_PLANES = 3;
+
+// Cell accumulators of one volume: [X+2][Y+2][Z+3], element (x + 1, y + 1, z + 1)
+// for floors (x, y, z); `cells` is floor (-1, -1, -1).
+struct CellAccumulators {
+    float4 *cells;
+    int X, Y, Z;
+
+    // the cell of floors (x, y, z) in [-1, N]
+    __device__ __forceinline__ float4 *cell(int x, int y, int z) const
+    {
+        return cells + ((size_t)((x + 1) * (Y + 2) + y + 1) * (Z + ACC_PLANES) + (z + 1));
+    }
+};
+
+// One ray's additions: consecutive samples in one cell (half a step apart by
+// default, about 1.4 per cell) are summed in registers and added once.
+// CHECK: a sample whose floor lies outside [-1, N] touches no voxel.
+template <bool CHECK>
+struct CellScatter {
+    const CellAccumulators &acc;
+    float4 *cur;
+    float4 lo, hi;  // at z, at z + 1
+
+    __device__ __forceinline__ explicit CellScatter(const CellAccumulators &a)
+        : acc(a), cur(nullptr), lo(make_float4(0.0f, 0.0f, 0.0f, 0.0f)), hi(lo)
+    {
+    }
+    __device__ __forceinline__ void flush()
+    {
+        if (!cur) return;
+        atomicAdd(cur, lo);
+        atomicAdd(cur + 1, hi);
+    }
+    __device__ __forceinline__ void add(float x, float y, float z, float val)
+    {
+        const FloorFrac fx = floor_frac(x), fy = floor_frac(y), fz = floor_frac(z);
+        if (CHECK && ((unsigned)(fx.i + 1) > (unsigned)(acc.X + 1) || (unsigned)(fy.i + 1) > (unsigned)(acc.Y + 1) ||
+                      (unsigned)(fz.i + 1) > (unsigned)(acc.Z + 1)))
+            return;
+        float4 *c = acc.cell(fx.i, fy.i, fz.i);
+        if (c != cur) {
+            flush();
+            cur = c;
+            lo = hi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        // weights of lerp_ref(a, b, t) = a (1 - t) + b t
+        const float h = val * fz.f, l = val * (1.0f - fz.f);
+        const float ty0 = 1.0f - fy.f, tx0 = 1.0f - fx.f;
+        const float w00 = ty0 * tx0, w10 = ty0 * fx.f, w01 = fy.f * tx0, w11 = fy.f * fx.f;
+        lo.x = fmaf(l, w00, lo.x), lo.y = fmaf(l, w10, lo.y), lo.z = fmaf(l, w01, lo.z), lo.w = fmaf(l, w11, lo.w);
+        hi.x = fmaf(h, w00, hi.x), hi.y = fmaf(h, w10, hi.y), hi.z = fmaf(h, w01, hi.z), hi.w = fmaf(h, w11, hi.w);
+    }
+};
+
+template <bool CHECK>
+__device__ __forceinline__ void scatter_ray(const ConeRay &ray, float step, float y, const CellAccumulators &acc)
+{
+    CellScatter<CHECK> s(acc);
+    cone_ray_weights(ray, step, [&](float px, float py, float pz, float w) { s.add(px, py, pz, y * w); });
+    s.flush();
+}
+
+// Grid: ray_block order (cone_ray.cuh).  z mode: a warp is 32 consecutive v at
+// one u, its sinogram values staged through shared memory; else 32
+// consecutive u.
+template <typename T>
+__global__ void __launch_bounds__(MB_X *MB_Y)
+    cone_scatter_cells_kernel(const T *__restrict__ sino, CellAccumulators acc, const ConeFpView *__restrict__ views,
+                              const float *__restrict__ step_ptr, const float *__restrict__ spacing_ptr, int W, int H,
+                              int n_proj, int g)
+{
+    __shared__ float tile[MB_Y][MB_X + 1];
+    const RayBlock rb = ray_block(blockIdx.x, W, H, n_proj);
+    const ConeFpView &view = views[(size_t)g * n_proj + rb.p];
+    const T *img = sino + (size_t)rb.p * H * (size_t)W;
+    int u, v;
+    float y = 0.0f;
+    if (view_is_z_mode(view)) {
+        const int t = threadIdx.y * MB_X + threadIdx.x;
+        const int iv = rb.tile_v * 32 + t / MB_Y, iu = rb.tile_u * 32 + rb.sub * MB_Y + t % MB_Y;
+        tile[t % MB_Y][t / MB_Y] = iu < W && iv < H ? load_as_float(img + (size_t)iv * W + iu) : 0.0f;
+        __syncthreads();
+        u = rb.tile_u * 32 + rb.sub * MB_Y + threadIdx.y;
+        v = rb.tile_v * 32 + threadIdx.x;
+        y = tile[threadIdx.y][threadIdx.x];
+    } else {
+        u = rb.tile_u * 32 + threadIdx.x;
+        v = rb.tile_v * 32 + rb.sub * MB_Y + threadIdx.y;
+        if (u < W && v < H) y = load_as_float(img + (size_t)v * W + u);
+    }
+    if (u >= W || v >= H || y == 0.0f || !in_footprint(view, u, v)) return;
+    const float step = step_ptr[g];
+    const ConeRay ray = cone_ray_setup(view, u, v, acc.X, acc.Y, acc.Z, 0.0, step, spacing_ptr[g * 3 + 2],
+                                       spacing_ptr[g * 3 + 1], spacing_ptr[g * 3 + 0]);
+    if (march_inside(ray, acc.X, acc.Y, acc.Z))
+        scatter_ray<false>(ray, step, y, acc);
+    else
+        scatter_ray<true>(ray, step, y, acc);
+}
+
+// The volume from its cell accumulators: a 32 (x) x 32 (z) tile of one y per
+// block, read along z and written along x.
+__global__ void __launch_bounds__(256) gather_cells_kernel(const float4 *__restrict__ cells, float *__restrict__ vol,
+                                                           int X, int Y, int Z)
+{
+    __shared__ float tile[32][33];
+    const int x0 = blockIdx.x * 32, z0 = blockIdx.z * 32, y = blockIdx.y;
+    const size_t s_y = Z + ACC_PLANES, s_x = s_y * (Y + 2);
+    const int z = z0 + threadIdx.x;
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int x = x0 + k;
+        if (x < X && z < Z) {
+            const float4 *c = cells + (x + 1) * s_x + (y + 1) * s_y + (z + 1);
+            tile[k][threadIdx.x] = (__ldg(c).x + __ldg(c - s_x).y) + (__ldg(c - s_y).z + __ldg(c - s_x - s_y).w);
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int x = x0 + threadIdx.x, zz = z0 + k;
+        if (x < X && zz < Z) vol[((size_t)zz * Y + y) * X + x] = tile[threadIdx.x][k];
+    }
+}
+
+template <typename T>
+cudaError_t scatter_cells(const void *sinogram, float *volume, const Dims3D &d, const ConeFpView *views,
+                          const float *step, const float *spacing, void *cells, cudaStream_t stream)
+{
+    const CellAccumulators acc{(float4 *)cells, d.vol_x, d.vol_y, d.vol_z};
+    const size_t voxels = (size_t)d.vol_z * d.vol_y * d.vol_x, pixels = (size_t)d.n_proj * d.det_h * d.det_w;
+    const dim3 block(MB_X, MB_Y), ggrid((d.vol_x + 31) / 32, d.vol_y, (d.vol_z + 31) / 32);
+    for (int b = 0; b < d.batch; ++b) {
+        cudaError_t e = cudaMemsetAsync(cells, 0, cone_scatter_cells_bytes(d.vol_z, d.vol_y, d.vol_x), stream);
+        if (e != cudaSuccess) return e;
+        cone_scatter_cells_kernel<T><<<ray_block_count(d.det_w, d.det_h, d.n_proj), block, 0, stream>>>(
+            (const T *)sinogram + b * pixels, acc, views, step, spacing, d.det_w, d.det_h, d.n_proj,
+            d.geom_batch == 1 ? 0 : b);
+        gather_cells_kernel<<<ggrid, dim3(32, 8), 0, stream>>>((const float4 *)cells, volume + b * voxels, d.vol_x,
+                                                               d.vol_y, d.vol_z);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 }  // namespace
+
+bool cone_ray_grid_fits(int det_w, int det_h, int n_proj)
+{
+    return ray_blocks_fit(det_w, det_h, n_proj);
+}
+
+size_t cone_scatter_cells_bytes(int vol_z, int vol_y, int vol_x)
+{
+    // cells are indexed with 32-bit columns, y is a grid dimension
+    if (vol_y > 65535 || (long long)(vol_x + 2) * (vol_y + 2) >= (1LL << 31)) return 0;
+    return (size_t)(vol_x + 2) * (vol_y + 2) * (vol_z + ACC_PLANES) * sizeof(float4);
+}
+
+cudaError_t launch_cone_scatter_cells(const void *sinogram, float *volume, int in_dtype, const Dims3D &d,
+                                      const ConeFpView *views, const float *step, const float *spacing, void *cells,
+                                      cudaStream_t stream)
+{
+    return dispatch_dtypes(in_dtype, PYRONN_FLOAT32, [&](auto tin, auto) {
+        return scatter_cells<typename decltype(tin)::type>(sinogram, volume, d, views, step, spacing, cells, stream);
+    });
+}
 
 cudaError_t launch_cone_scatter(const void *sinogram, float *volume, int in_dtype, const Dims3D &d,
                                 const ConeFpView *views, const float *step, const float *spacing,

@@ -85,6 +85,14 @@ cudaError_t launch_fdk_filter_tc(const void *in, void *out, int in_dtype, int ou
 // clears it when set); synchronises the stream
 cudaError_t fdk_tc_error(cudaStream_t stream, unsigned *device_error);
 
+// whether the ray block order's grid (cone_ray.cuh) fits one launch
+bool cone_ray_grid_fits(int det_w, int det_h, int n_proj);
+// the same over cell accumulators (`cells`: device, cone_scatter_cells_bytes,
+// 16-byte aligned; 0 bytes where they do not apply)
+size_t cone_scatter_cells_bytes(int vol_z, int vol_y, int vol_x);
+cudaError_t launch_cone_scatter_cells(const void *sinogram, float *volume, int in_dtype, const Dims3D &d,
+                                      const ConeFpView *views, const float *step, const float *spacing, void *cells,
+                                      cudaStream_t stream);
 cudaError_t launch_cone_scatter(const void *sinogram, float *volume, int in_dtype, const Dims3D &d,
                                 const ConeFpView *views, const float *step, const float *spacing,
                                 cudaStream_t stream);

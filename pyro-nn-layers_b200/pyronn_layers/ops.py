@@ -310,6 +310,17 @@ def _run_2d(forward: bool, x: torch.Tensor, out_dims, geo: Geometry2D, out_dtype
     return out
 
 
+def _workspace(nbytes: int, device, least=None) -> torch.Tensor:
+    """A workspace of nbytes; where that does not fit the device's memory, one
+    of least() bytes (an op whose entry point accepts it, without its copies)."""
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        if least is None or least() >= nbytes:
+            raise
+        return torch.empty(least(), dtype=torch.uint8, device=device)
+
+
 def _run_cone(forward: bool, x: torch.Tensor, out_dims, geo: GeometryCone, hardware_interp: bool,
               out_dtype=None, workspace=None) -> torch.Tensor:
     batch = x.shape[0]
@@ -331,7 +342,9 @@ def _run_cone(forward: bool, x: torch.Tensor, out_dims, geo: GeometryCone, hardw
         ws_args = dims + [storage_code(x.dtype), int(bool(hardware_interp)), geo.g]
     ws_bytes = _capi.workspace_size(fn, *ws_args)
     if workspace is None or workspace.numel() < ws_bytes:
-        workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+        # a backprojection's query without a batch is its per-view part alone
+        least = None if forward else lambda: _capi.workspace_size(fn, 0, *ws_args[1:])
+        workspace = _workspace(ws_bytes, dev, least)
     with torch.cuda.device(dev):
         _capi.call(fn, x.data_ptr(), out.data_ptr(), storage_code(x.dtype), storage_code(od),
                    int(bool(hardware_interp)), *dims, *geo.pointers(), geo.g, workspace.data_ptr(),
@@ -348,12 +361,12 @@ def _run_matched(p: torch.Tensor, vol_dims, geo: GeometryCone) -> torch.Tensor:
     vol_z, vol_y, vol_x = vol_dims
     out = torch.empty((batch, vol_z, vol_y, vol_x), dtype=torch.float32, device=dev)
     fn = "pyronn_cone_backprojection3d_matched"
-    ws_bytes = _capi.workspace_size(fn, geo.g, n_proj)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+    ws_bytes = _capi.workspace_size(fn + "_cells", geo.g, n_proj, det_h, det_w, vol_z, vol_y, vol_x)
+    ws = _workspace(ws_bytes, dev, lambda: _capi.workspace_size(fn, geo.g, n_proj))
     with torch.cuda.device(dev):
         _capi.call(fn, p.data_ptr(), out.data_ptr(), storage_code(p.dtype), batch, n_proj, det_h, det_w, vol_z, vol_y,
                    vol_x, geo.volume_origin.data_ptr(), geo.volume_spacing.data_ptr(),
-                   geo.projection_matrices.data_ptr(), geo.step_size.data_ptr(), geo.g, ws.data_ptr(), ws_bytes,
+                   geo.projection_matrices.data_ptr(), geo.step_size.data_ptr(), geo.g, ws.data_ptr(), ws.numel(),
                    _stream(dev))
     return out
 

@@ -139,3 +139,41 @@ def test_cone_forward_fp32_cell_pitch(cuda):
     out = pl.cone_projection3d(t(vol, cuda), geo.detector_shape, *geo.args())
     ref = oracle.cone_projection3d(vol, geo.detector_shape, *geo.args())
     assert rel_l2(out.cpu().numpy(), ref) < 2e-5
+
+
+# ------------------------------------------------- matched cone backprojection
+
+
+def _tilted(geo, angle):
+    """The scan's projection matrices with the object turned about the y axis."""
+    c, s = np.cos(angle), np.sin(angle)
+    r = np.array([[c, 0, s, 0], [0, 1, 0, 0], [-s, 0, c, 0], [0, 0, 0, 1]])
+    return (geo.projection_matrices.astype(np.float64) @ r).astype(np.float32)
+
+
+@pytest.mark.parametrize("vol_shape,det,batch,tilt,dtype", [
+    ((1, 1, 1), (3, 3), 1, 0.0, torch.float32),
+    ((5, 33, 31), (9, 40), 2, 0.0, torch.bfloat16),
+    ((34, 20, 23), (40, 33), 3, 0.0, torch.float32),
+    ((20, 21, 22), (33, 31), 1, 0.5 * np.pi, torch.float32),  # detector rows along z: warps along u
+    ((20, 21, 22), (33, 31), 1, 0.4, torch.float16),
+])
+def test_matched_backprojection_cells(cuda, vol_shape, det, batch, tilt, dtype):
+    """The matched backprojection over cell accumulators, and with a workspace
+    of the per-view part alone (scattered into the volume), against the FP64
+    oracle: FP32 sums of FP32 weights, 1e-5 (as the backprojections)."""
+    geo = geometry.ConeBeam3D(vol_shape, (1.0, 0.9, 1.1), det, (1.3, 1.2), 7, 60.0, 100.0, step_size=0.5)
+    args = (geo.volume_origin, geo.volume_spacing, _tilted(geo, tilt), geo.step_size)
+    p = t(noise(21, (batch,) + geo.detector_shape), cuda, dtype)
+    ref = oracle.cone_backprojection3d_matched(p.float().cpu().numpy(), vol_shape, *args)
+    out = pl.cone_backprojection3d_matched(p, vol_shape, *args)
+    assert rel_l2(out.cpu().numpy(), ref) < 1e-5
+    g = pl.ops.GeometryCone(batch, cuda, *args, 1.0, geo.detector_shape[0])
+    n = _capi.workspace_size("pyronn_cone_backprojection3d_matched", g.g, geo.detector_shape[0])
+    ws = torch.empty(n, dtype=torch.uint8, device=cuda)
+    plain = torch.full_like(out, 7.0)
+    _capi.call("pyronn_cone_backprojection3d_matched", p.data_ptr(), plain.data_ptr(), pl.ops.storage_code(dtype),
+               batch, *geo.detector_shape, *vol_shape, g.volume_origin.data_ptr(), g.volume_spacing.data_ptr(),
+               g.projection_matrices.data_ptr(), g.step_size.data_ptr(), g.g, ws.data_ptr(), n,
+               torch.cuda.current_stream().cuda_stream)
+    assert rel_l2(plain.cpu().numpy(), ref) < 1e-5
