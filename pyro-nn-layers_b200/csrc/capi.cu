@@ -322,10 +322,10 @@ size_t pyronn_cone_backprojection3d_workspace_size(int batch, int n_proj, int de
     if (geom_batch <= 0 || n_proj <= 0 || !valid_dtype(in_dtype)) return 0;
     const size_t views = WS_HEADER + align_up((size_t)geom_batch * n_proj * sizeof(ConeBpView), 256);
     if (hardware_interp || batch <= 0 || det_h <= 0 || det_w <= 0) return views;
-    // 16-bit sinograms: room for the paired copy the TMA path reads (a
-    // workspace of `views` bytes alone is accepted, without the pairing)
+    // room for the copy of the sinogram the TMA path reads where it takes one
+    // (a workspace of `views` bytes alone is accepted, without the copy)
     const Dims3D d{batch, vol_z, vol_y, vol_x, n_proj, det_h, det_w, geom_batch};
-    return views + align_up(cone_bp_tma_paired_bytes(in_dtype, d), 256);
+    return views + align_up(cone_bp_tma_copy_bytes(in_dtype, d), 256);
 }
 
 int pyronn_workspace_error(const void *workspace, void *stream, int *device_error)
@@ -409,7 +409,7 @@ int pyronn_cone_backprojection3d(const void *sinogram, void *volume, int in_dtyp
     int st = check_cone(name, sinogram, volume, in_dtype, out_dtype, d, volume_origin, volume_spacing, projection_matrices,
                         step_size, projection_multiplier);
     if (st) return st;
-    // the views' part is required; the paired copy is used when it fits
+    // the views' part is required; the sinogram's copy is used when it fits
     const size_t need = WS_HEADER + align_up((size_t)geom_batch * n_proj * sizeof(ConeBpView), 256);
     if (!workspace || workspace_bytes < need)
         return fail(PYRONN_ERROR_WORKSPACE_TOO_SMALL, "%s: workspace of %zu bytes needed, %zu given", name, need,
@@ -428,12 +428,11 @@ int pyronn_cone_backprojection3d(const void *sinogram, void *volume, int in_dtyp
     e = launch_cone_bp_prepare(projection_matrices, volume_spacing, volume_origin, geom_batch, n_proj, views, s);
     if (e != cudaSuccess) return cuda_fail(e, "cone_backprojection3d: geometry preparation");
     if (!hardware_interp) {
-        if (cone_bp_tma_supported(sinogram, in_dtype, d)) {
-            const size_t pb = cone_bp_tma_paired_bytes(in_dtype, d);
-            void *paired = (pb > 0 && workspace_bytes >= need + pb) ? (char *)workspace + need : nullptr;
-            e = launch_cone_bp_tma(sinogram, volume, in_dtype, out_dtype, d, views, projection_multiplier, err,
-                                   paired, s);
-        }
+        const size_t cb = cone_bp_tma_copy_bytes(in_dtype, d);
+        void *copy = (cb > 0 && workspace_bytes >= need + cb) ? (char *)workspace + need : nullptr;
+        if (cone_bp_tma_supported(sinogram, in_dtype, d, copy != nullptr))
+            e = launch_cone_bp_tma(sinogram, volume, in_dtype, out_dtype, d, views, projection_multiplier, err, copy,
+                                   s);
         else
             e = launch_cone_bp(sinogram, volume, in_dtype, out_dtype, d, -1, views, projection_multiplier, 0, s);
         if (e != cudaSuccess) return cuda_fail(e, name);

@@ -23,6 +23,11 @@
 // same bits).  512^3 workload: backprojection 32.5 -> 31.8 ms, the pairing
 // pass (1.1 GB written) included.
 //
+// Detector rows that are no multiple of 16 bytes, which TMA cannot address,
+// are likewise copied to rows of such a pitch first (the paired copy where
+// that pays, else a plain one): 181 x 203 x 219 voxels, 271 views of 287 x 347 in
+// BF16 take 2.2 ms, the copy included, against 6.3 ms in the direct-gather kernel.
+//
 // Exactness: the tap indices and weights are computed exactly as the direct
 // path computes them (floor of u/w, frac), only the texel source differs.  TMA
 // zero-fills out-of-range texels, which equals the reference's semantics for
@@ -482,13 +487,49 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// A copy of the sinogram's rows (any storage type) at a pitch of Wp elements,
+// a multiple of 16 bytes.  Grid as the pairing's; a thread writes 16 bytes.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    pitch_sinogram_kernel(const T *__restrict__ sino, T *__restrict__ dst, int W, int Wp, long long rows)
+{
+    constexpr int N = 16 / (int)sizeof(T);
+    const int x = (blockIdx.x * 256 + threadIdx.x) * N;
+    if (x >= Wp) return;
+    for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
+        union {
+            T v[N];
+            uint4 q;
+        } out;
+#pragma unroll
+        for (int k = 0; k < N; ++k) out.v[k] = x + k < W ? sino[r * W + x + k] : T(0.0f);
+        *reinterpret_cast<uint4 *>(dst + r * Wp + x) = out.q;
+    }
+}
+
+inline int pitched_row(int W, size_t elem)
+{
+    const int n = 16 / (int)elem;
+    return (W + n - 1) / n * n;
+}
+
 inline int paired_row(int W)
 {
     return (W + 1 + 3) / 4 * 4;
 }
 
+// whether a 16-bit sinogram's paired copy pays: the pairing pass costs about a
+// read and two writes of the sinogram and saves a shared-memory load per tap
+// pair, worth it when a detector pixel serves many voxel updates (512^3 on
+// 1024 x 768: 171, 31.8 against 32.5 ms; 256^3 on 512^2: 64, 4.26 against 4.08 ms)
+inline bool pairing_pays(int in_dtype, const Dims3D &d)
+{
+    return dtype_size(in_dtype) == 2 && (long long)d.vol_x * d.vol_y * d.vol_z >= 100LL * d.det_h * d.det_w;
+}
+
+// `pitch`: elements between the staged rows
 template <typename Tin, typename Tout, bool PAIRED>
-cudaError_t launch_kernel(const void *sinogram, const void *staged, void *volume, const Dims3D &d,
+cudaError_t launch_kernel(const void *sinogram, const void *staged, int pitch, void *volume, const Dims3D &d,
                           const ConeBpView *views, const float *mult, unsigned *err, int starve_last_pass,
                           cudaStream_t stream)
 {
@@ -496,10 +537,10 @@ cudaError_t launch_kernel(const void *sinogram, const void *staged, void *volume
     if (!enc) return cudaErrorNotSupported;
     using L = BoxLayout<Tin, PAIRED>;
     using E = typename L::E;
-    const cuuint64_t row = PAIRED ? (cuuint64_t)paired_row(d.det_w) : (cuuint64_t)d.det_w;
+    const cuuint64_t row = PAIRED ? (cuuint64_t)pitch : (cuuint64_t)d.det_w;
     CUtensorMap map;
     const cuuint64_t dims[3] = {row, (cuuint64_t)d.det_h, (cuuint64_t)d.n_proj * d.batch};
-    const cuuint64_t strides[2] = {row * sizeof(E), row * d.det_h * sizeof(E)};
+    const cuuint64_t strides[2] = {pitch * sizeof(E), (cuuint64_t)pitch * d.det_h * sizeof(E)};
     const cuuint32_t box[3] = {(cuuint32_t)L::W, BOX_H, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType type = PAIRED ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : tma_type<Tin>();
@@ -526,34 +567,46 @@ cudaError_t launch_kernel(const void *sinogram, const void *staged, void *volume
 }
 
 template <typename Tin, typename Tout>
-cudaError_t launch_typed(const void *sinogram, void *volume, const Dims3D &d, const ConeBpView *views,
-                         const float *mult, unsigned *err, int starve_last_pass, void *paired, cudaStream_t stream)
+cudaError_t launch_typed(const void *sinogram, void *volume, int in_dtype, const Dims3D &d, const ConeBpView *views,
+                         const float *mult, unsigned *err, int starve_last_pass, void *copy, cudaStream_t stream)
 {
+    const long long rows = (long long)d.batch * d.n_proj * d.det_h;
+    const unsigned ygrid = (unsigned)(rows < 65535 ? rows : 65535);
     if constexpr (sizeof(Tin) == 2) {
-        if (paired) {
+        if (copy && pairing_pays(in_dtype, d)) {
             const int Wp = paired_row(d.det_w);
-            const long long rows = (long long)d.batch * d.n_proj * d.det_h;
-            const dim3 pgrid((unsigned)((Wp + 255) / 256), (unsigned)(rows < 65535 ? rows : 65535));
-            pair_sinogram_kernel<Tin><<<pgrid, 256, 0, stream>>>((const Tin *)sinogram, (unsigned *)paired, d.det_w,
-                                                                 Wp, rows);
+            pair_sinogram_kernel<Tin><<<dim3((unsigned)((Wp + 255) / 256), ygrid), 256, 0, stream>>>(
+                (const Tin *)sinogram, (unsigned *)copy, d.det_w, Wp, rows);
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
-            return launch_kernel<Tin, Tout, true>(sinogram, paired, volume, d, views, mult, err, starve_last_pass,
+            return launch_kernel<Tin, Tout, true>(sinogram, copy, Wp, volume, d, views, mult, err, starve_last_pass,
                                                   stream);
         }
     }
-    return launch_kernel<Tin, Tout, false>(sinogram, sinogram, volume, d, views, mult, err, starve_last_pass, stream);
+    if (copy) {
+        const int Wp = pitched_row(d.det_w, sizeof(Tin));
+        const int chunks = Wp / (16 / (int)sizeof(Tin));
+        pitch_sinogram_kernel<Tin><<<dim3((unsigned)((chunks + 255) / 256), ygrid), 256, 0, stream>>>(
+            (const Tin *)sinogram, (Tin *)copy, d.det_w, Wp, rows);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        return launch_kernel<Tin, Tout, false>(sinogram, copy, Wp, volume, d, views, mult, err, starve_last_pass,
+                                               stream);
+    }
+    return launch_kernel<Tin, Tout, false>(sinogram, sinogram, d.det_w, volume, d, views, mult, err, starve_last_pass,
+                                           stream);
 }
 
 }  // namespace
 
-// The TMA path needs 16-byte aligned sinogram rows and base, and a grid that
-// fits one launch; the caller falls back to the direct kernel otherwise.
-bool cone_bp_tma_supported(const void *sinogram, int in_dtype, const Dims3D &d)
+// The TMA path needs 16-byte aligned rows and base (the sinogram's, or a
+// copy's) and a grid that fits one launch; the caller falls back to the direct
+// kernel otherwise.
+bool cone_bp_tma_supported(const void *sinogram, int in_dtype, const Dims3D &d, bool copy)
 {
     const size_t e = dtype_size(in_dtype);
-    if (e == 0 || ((uintptr_t)sinogram % 16) != 0) return false;
-    if (((size_t)d.det_w * e) % 16 != 0) return false;
+    if (e == 0) return false;
+    if (!copy && (((uintptr_t)sinogram % 16) != 0 || ((size_t)d.det_w * e) % 16 != 0)) return false;
     const long long zb = (d.vol_z + TB_Z - 1) / TB_Z;
     if (zb * d.batch > 65535 || (d.vol_y + TB_Y - 1) / TB_Y > 65535) return false;
     if ((long long)d.n_proj * d.batch >= (1LL << 31)) return false;
@@ -569,26 +622,23 @@ void cone_bp_tma_starve_last_pass(int enable)
     g_starve_last_pass.store(enable ? 1 : 0);
 }
 
-size_t cone_bp_tma_paired_bytes(int in_dtype, const Dims3D &d)
+size_t cone_bp_tma_copy_bytes(int in_dtype, const Dims3D &d)
 {
-    // the pairing pass costs about a read and two writes of the sinogram and
-    // saves a shared-memory load per tap pair: it pays when a detector pixel
-    // serves many voxel updates (512^3 on 1024 x 768: 171, 31.8 against
-    // 32.5 ms; 256^3 on 512^2: 64, 4.26 against 4.08 ms)
-    if (dtype_size(in_dtype) != 2) return 0;
-    if ((long long)d.vol_x * d.vol_y * d.vol_z < 100LL * d.det_h * d.det_w) return 0;
-    return (size_t)d.batch * d.n_proj * d.det_h * (size_t)paired_row(d.det_w) * sizeof(unsigned);
+    const size_t e = dtype_size(in_dtype), rows = (size_t)d.batch * d.n_proj * d.det_h;
+    if (e == 0) return 0;
+    if (pairing_pays(in_dtype, d)) return rows * (size_t)paired_row(d.det_w) * sizeof(unsigned);
+    return ((size_t)d.det_w * e) % 16 != 0 ? rows * (size_t)pitched_row(d.det_w, e) * e : 0;
 }
 
 cudaError_t launch_cone_bp_tma(const void *sinogram, void *volume, int in_dtype, int out_dtype, const Dims3D &d,
-                               const ConeBpView *views, const float *mult, unsigned *err, void *paired,
+                               const ConeBpView *views, const float *mult, unsigned *err, void *copy,
                                cudaStream_t stream)
 {
     const int starve = g_starve_last_pass.load();
     return dispatch_dtypes(in_dtype, out_dtype, [&](auto tin, auto tout) {
         using Tin = typename decltype(tin)::type;
         using Tout = typename decltype(tout)::type;
-        return launch_typed<Tin, Tout>(sinogram, volume, d, views, mult, err, starve, paired, stream);
+        return launch_typed<Tin, Tout>(sinogram, volume, in_dtype, d, views, mult, err, starve, copy, stream);
     });
 }
 

@@ -98,14 +98,15 @@ cudaError_t launch_cone_scatter(const void *sinogram, float *volume, int in_dtyp
                                 cudaStream_t stream);
 
 // TMA-staged software backprojector (cone_bp_tma.cu); err = device error flag
-bool cone_bp_tma_supported(const void *sinogram, int in_dtype, const Dims3D &d);
-// Bytes of the paired copy of a 16-bit sinogram (0 for FP32, or where the
-// copy does not pay): with it the TMA backprojector stages 32-bit tap pairs,
-// one shared-memory load per lerp.
-size_t cone_bp_tma_paired_bytes(int in_dtype, const Dims3D &d);
-// `paired` (device, 16-byte aligned, cone_bp_tma_paired_bytes) or null.
+// (copy: a copy of cone_bp_tma_copy_bytes will be given)
+bool cone_bp_tma_supported(const void *sinogram, int in_dtype, const Dims3D &d, bool copy);
+// Bytes of the copy of the sinogram the TMA backprojector stages its boxes
+// from: 32-bit tap pairs of a 16-bit sinogram where that pays (one shared-memory
+// load per lerp), rows at a 16-byte pitch where the sinogram's are none; else 0.
+size_t cone_bp_tma_copy_bytes(int in_dtype, const Dims3D &d);
+// `copy` (device, 16-byte aligned, cone_bp_tma_copy_bytes) or null.
 cudaError_t launch_cone_bp_tma(const void *sinogram, void *volume, int in_dtype, int out_dtype, const Dims3D &d,
-                               const ConeBpView *views, const float *mult, unsigned *err, void *paired,
+                               const ConeBpView *views, const float *mult, unsigned *err, void *copy,
                                cudaStream_t stream);
 // testing hook (pyronn_debug_starve_tma_wait): while enabled, the last pass of
 // every TMA backprojector block issues no copies and expects bytes that never

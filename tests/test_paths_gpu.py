@@ -177,3 +177,36 @@ def test_matched_backprojection_cells(cuda, vol_shape, det, batch, tilt, dtype):
                g.projection_matrices.data_ptr(), g.step_size.data_ptr(), g.g, ws.data_ptr(), n,
                torch.cuda.current_stream().cuda_stream)
     assert rel_l2(plain.cpu().numpy(), ref) < 1e-5
+
+
+# -------------------------------------------------------- cone backprojection
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vol_shape,det,pitch,batch", [
+    ((9, 10, 33), (7, 1), 3.0, 1),      # one-pixel rows
+    ((17, 21, 40), (31, 37), 1.6, 2),   # rows of no multiple of 16 bytes, batch of two
+    ((33, 40, 45), (29, 129), 0.7, 1),  # a row one element past a multiple of 16 bytes
+    ((48, 50, 52), (23, 29), 3.1, 1),   # the same with more than 100 voxels per pixel (16-bit: paired copy)
+])
+def test_cone_backprojection_unaligned_rows(cuda, vol_shape, det, pitch, batch, dtype):
+    """Detector rows TMA cannot address: over a pitched (or paired) copy given
+    the queried workspace, by direct gathers given the views' part alone; both
+    against the oracle.  The second sinogram starts off a 16-byte boundary."""
+    geo = geometry.ConeBeam3D(vol_shape, (1.0, 0.9, 1.1), det, (pitch, pitch), 9, 160.0, 260.0)
+    sino = t(noise(31, (batch,) + geo.detector_shape), cuda, dtype)
+    shifted = torch.empty(sino.numel() + 1, device=cuda, dtype=dtype)[1:].view(sino.shape)
+    shifted.copy_(sino)
+    ref = oracle.cone_backprojection3d(sino.float().cpu().numpy(), vol_shape, *geo.args())
+    gc = pl.ops.GeometryCone(batch, cuda, *geo.args(), geo.detector_shape[0])
+    code = pl.ops.storage_code(dtype)
+    query = ("pyronn_cone_backprojection3d", batch, *geo.detector_shape, *vol_shape, code, 0, gc.g)
+    full, views = _capi.workspace_size(*query), _capi.workspace_size(query[0], 0, *query[2:])
+    assert full > views
+    for p in (sino, shifted):
+        for nbytes in (full, views):
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=cuda)
+            out = torch.full((batch,) + vol_shape, 7.0, device=cuda)
+            _capi.call(query[0], p.data_ptr(), out.data_ptr(), code, 0, 0, batch, *geo.detector_shape, *vol_shape,
+                       *gc.pointers(), gc.g, ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
+            assert rel_l2(out.cpu().numpy(), ref) < 1e-5
