@@ -8,7 +8,8 @@
 // linearly along the row: q[j] = tau * sum_k h[j - k] g[k], tau the column
 // pitch.  FP32 arithmetic, storage types as the projector ops.
 //
-// Kernel: direct convolution on the FP32 pipes.  A block holds `rows` whole
+// Rows of up to 2048 pixels take the transforms of fdk_fft.cu.  Wider ones
+// the kernel here: direct convolution on the FP32 pipes.  A block holds `rows` whole
 // detector rows and the taps in shared memory; each thread computes 16
 // consecutive outputs of one row with a sliding window of 16 taps in
 // registers: per input sample k, one tap load (the window's new element),
@@ -144,15 +145,10 @@ cudaError_t launch_fdk_filter(const void *in, void *out, int in_dtype, int out_d
                               int W, float sdd, float dv, float du, float cv, float cu, int kind, int weight_output,
                               cudaStream_t stream)
 {
-    // the tensor-core kernel reads a row's inputs from every output tile of
-    // it, so it needs distinct input and output buffers; in-place calls take
-    // the CUDA-core kernel, which holds whole rows in shared memory
-    const char *ib = (const char *)in, *ob = (const char *)out;
-    const size_t n = (size_t)rows * (size_t)W;
-    const bool overlap = ib < ob + n * dtype_size(out_dtype) && ob < ib + n * dtype_size(in_dtype);
-    if (fdk_tc_supported(rows, W, in, out) && !overlap)
-        return launch_fdk_filter_tc(in, out, in_dtype, out_dtype, rows, det_h, W, sdd, dv, du, cv, cu, kind,
-                                    weight_output, stream);
+    // the direct sums take O(W^2) per row: only rows wider than the transforms'
+    if (fdk_fft_supported(W))
+        return launch_fdk_filter_fft(in, out, in_dtype, out_dtype, rows, det_h, W, sdd, dv, du, cv, cu, kind,
+                                     weight_output, stream);
     const int chunks = (W + FB - 1) / FB;
     const int tpr = (chunks + 31) / 32 * 32;  // threads per row, a warp multiple
     const int rpb = 256 / tpr > 0 ? 256 / tpr : 1;

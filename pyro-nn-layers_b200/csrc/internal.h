@@ -75,15 +75,11 @@ cudaError_t launch_cone_fp_padded(const void *volume, void *sinogram, int in_dty
 cudaError_t launch_fdk_filter(const void *in, void *out, int in_dtype, int out_dtype, long long rows, int det_h,
                               int W, float sdd, float dv, float du, float cv, float cu, int kind, int weight_output,
                               cudaStream_t stream);
-// the same on the tensor cores (fdk_tc.cu): rows of at most 2048 pixels, a
-// multiple of 4, 16-byte aligned buffers, at most 65535 * 128 rows
-bool fdk_tc_supported(long long rows, int W, const void *in, const void *out);
-cudaError_t launch_fdk_filter_tc(const void *in, void *out, int in_dtype, int out_dtype, long long rows, int det_h,
-                                 int W, float sdd, float dv, float du, float cv, float cu, int kind,
-                                 int weight_output, cudaStream_t stream);
-// reads the filter's sticky device error word on the current device (and
-// clears it when set); synchronises the stream
-cudaError_t fdk_tc_error(cudaStream_t stream, unsigned *device_error);
+// the same by fast Fourier transforms (fdk_fft.cu): rows of at most 2048 pixels
+bool fdk_fft_supported(int W);
+cudaError_t launch_fdk_filter_fft(const void *in, void *out, int in_dtype, int out_dtype, long long rows, int det_h,
+                                  int W, float sdd, float dv, float du, float cv, float cu, int kind,
+                                  int weight_output, cudaStream_t stream);
 
 // whether the ray block order's grid (cone_ray.cuh) fits one launch
 bool cone_ray_grid_fits(int det_w, int det_h, int n_proj);

@@ -10,7 +10,7 @@ import torch
 
 import oracle
 import pyronn_layers as pl
-from pyronn_layers import _capi, geometry
+from pyronn_layers import _capi, fbp, geometry
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -210,3 +210,44 @@ def test_cone_backprojection_unaligned_rows(cuda, vol_shape, det, pitch, batch, 
             _capi.call(query[0], p.data_ptr(), out.data_ptr(), code, 0, 0, batch, *geo.detector_shape, *vol_shape,
                        *gc.pointers(), gc.g, ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
             assert rel_l2(out.cpu().numpy(), ref) < 1e-5
+
+
+# ------------------------------------------------------------------ ramp filter
+
+
+@pytest.mark.parametrize("filt", ["ram-lak", "shepp-logan"])
+@pytest.mark.parametrize("rows,width", [
+    ((1, 1, 1), 1), ((1, 3, 5), 2),          # tiny rows; an odd number of rows
+    ((2, 9, 1), 255), ((1, 3, 40), 256),     # transforms of 512 points, the widest exactly half
+    ((1, 5, 13), 257), ((1, 2, 7), 512),     # 1024 points
+    ((1, 1, 11), 513), ((1, 2, 3), 1024),    # 2048 points
+    ((1, 1, 3), 1025), ((1, 1, 3), 2047), ((1, 1, 2), 2048),  # 4096 points
+    ((1, 1, 3), 2049),                       # direct sums
+])
+def test_filter_widths(cuda, rows, width, filt):
+    """The ramp filter at the edges of its transform lengths against the FP64
+    oracle: 1e-5, as test_fbp_gpu.py; rows of very different magnitude are
+    each held to it."""
+    b, n, h = rows
+    p = noise(width, rows + (width,))
+    p[:, :, ::2] *= np.float32(1e-6)
+    out = fbp.fdk_filter(t(p, cuda), 800.0, (1.1, 0.7), None, filt).cpu().numpy()
+    kind = oracle.filters.RAM_LAK if filt == "ram-lak" else oracle.filters.SHEPP_LOGAN
+    ref = oracle.fdk_filter(p, 800.0, 1.1, 0.7, (h - 1) / 2, (width - 1) / 2, kind)
+    for i in np.ndindex(*rows):
+        assert rel_l2(out[i], ref[i]) < 1e-5
+
+
+def test_filter_keeps_rows_apart(cuda):
+    """Infinities and NaNs in a row make that row NaN and leave the others as
+    they are; a row of zeros stays zeros."""
+    p = noise(3, (1, 1, 8, 300))
+    clean = fbp.fdk_filter(t(p, cuda), 500.0, (1.0, 1.0))
+    q = p.copy()
+    q[0, 0, 1, 17], q[0, 0, 4, 299], q[0, 0, 6] = np.inf, np.nan, 0.0
+    out = fbp.fdk_filter(t(q, cuda), 500.0, (1.0, 1.0))
+    for r in (0, 2, 3, 5, 7):
+        assert torch.equal(out[0, 0, r], clean[0, 0, r]) or rel_l2(out[0, 0, r].cpu().numpy(),
+                                                                   clean[0, 0, r].cpu().numpy()) < 1e-6
+    assert torch.isnan(out[0, 0, 1]).all() and torch.isnan(out[0, 0, 4]).all()
+    assert (out[0, 0, 6] == 0).all()
