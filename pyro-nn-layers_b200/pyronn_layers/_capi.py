@@ -7,6 +7,7 @@ library is missing or fails to load, every op raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 LIB_NAME = "libpyronn_b200.so"
@@ -129,13 +130,14 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
 
 def call(name: str, *args) -> None:
     """Calls an entry point and raises PyronnError on a non-success status."""
-    lib = load()
+    lib = _lib or load()
     status = getattr(lib, name)(*args)
     if status != SUCCESS:
         detail = lib.pyronn_last_error().decode("utf-8", "replace")
         raise PyronnError(name, status, detail)
 
 
+@functools.lru_cache(maxsize=1024)
 def workspace_size(name: str, *args: int) -> int:
     """Workspace bytes of an entry point (``pyronn_projection2d`` for both 2D
     forward ops); args as the C query takes them."""
