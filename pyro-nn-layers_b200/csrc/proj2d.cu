@@ -270,11 +270,19 @@ __device__ __forceinline__ float sum_cells(const Ray2D &ray, float a, int kmax, 
         sign = ray.gm < 0.0f ? -1 : 1;
         off = -__reduce_min_sync(mask, alive ? sign * p.mi : 0x7fffffff);
     }
+    // AHEAD: a visit's taps are loaded while the previous visit is computed
+    // (one slice: 5 % faster; two or more have no registers for it: 0.65 -> 0.90 ms
+    // on three 387 x 451 fan slices)
+    constexpr bool AHEAD = NS == 1;
+    float4 w[NS], ahead[AHEAD ? NS : 1];
+    if (AHEAD && alive) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) ahead[s] = taps(p.mi, p.ni, s);
+    }
     for (int column = COLS - 1; alive; column += COLS) {
         while (alive && (!Taps::ALIGN_COLUMNS || sign * p.mi + off <= column)) {
-            float4 w[NS];
 #pragma unroll
-            for (int s = 0; s < NS; ++s) w[s] = taps(p.mi, p.ni, s);
+            for (int s = 0; s < NS; ++s) w[s] = AHEAD ? ahead[s] : taps(p.mi, p.ni, s);
             // samples of this visit: up to the nearer face or the run's end,
             // at least one (ceiling by a sum rounded up, as floor_frac's;
             // exact below 2^22, and nf is)
@@ -287,6 +295,10 @@ __device__ __forceinline__ float sum_cells(const Ray2D &ray, float a, int kmax, 
             jf += L;
             if (jf >= nf) next_run();
             p = run.at(jf);
+            if (AHEAD && alive) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) ahead[s] = taps(p.mi, p.ni, s);
+            }
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
                 const float2 lo = pair(w[s].x, w[s].y), hi = pair(w[s].z, w[s].w);
@@ -338,8 +350,6 @@ __device__ __forceinline__ void march_ray(const Ray2D &ray, const Taps &taps, un
     int kmax = march2d_max_iter(ray.a, ray.am, ray.step), k0 = 0;
     float a = ray.a;
     if (SEG > 1) {
-        float b;
-        const int n = samples_before(ray, ray.am, kmax, b);
         // band boundaries in the ray's direction; neighbouring bands evaluate
         // the same bound, so every sample falls in one band (a bound that is
         // not a number, or behind the ray, leaves the earlier band empty)
@@ -347,11 +357,11 @@ __device__ __forceinline__ void march_ray(const Ray2D &ray, const Taps &taps, un
             const float m = (float)extent * ((float)(ray.gm < 0.0f ? SEG - i : i) / (float)SEG);
             return fminf((m - ray.bm) / ray.gm, ray.am);
         };
-        int k1 = n;
         if (seg > 0) k0 = samples_before(ray, bound(seg), kmax, a);
-        if (seg < SEG - 1) k1 = samples_before(ray, bound(seg + 1), kmax, b);
+        float b;  // the alpha after the band: not below the exit if the band holds the last sample
+        const int k1 = samples_before(ray, seg < SEG - 1 ? bound(seg + 1) : ray.am, kmax, b);
+        holds_last = k1 > k0 && (!(b < ray.am) || k1 == kmax);
         kmax = max(k1 - k0, 0);
-        holds_last = kmax > 0 && k1 == n;
     } else {
         holds_last = a < ray.am && kmax > 0;
     }
@@ -381,7 +391,7 @@ __global__ void __launch_bounds__(FP2_BLOCK, NS == 4 ? 7 : 8)
                         int X, int Y, int W, int n_proj, int batch, int geom_batch)
 {
     constexpr int RAYS = FP2_BLOCK / SEG;  // rays per block
-    static_assert(SEG == 1 || RAYS == 32, "a segment per warp");
+    static_assert(RAYS % 32 == 0, "warps within a segment");
     static_assert(SEG == 1 || NS == 1, "ranges take one slice");
     const int lane = threadIdx.x % RAYS, seg = threadIdx.x / RAYS;
     const int u = blockIdx.x * RAYS + lane;
