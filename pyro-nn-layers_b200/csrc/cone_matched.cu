@@ -103,36 +103,43 @@ template <bool CHECK>
 struct CellScatter {
     const CellAccumulators &acc;
     float4 *cur;
-    float4 lo, hi;  // at z, at z + 1
+    float2 lo[2], hi[2];  // at z, at z + 1: the (x0, x1) pairs of y0 and y1
 
-    __device__ __forceinline__ explicit CellScatter(const CellAccumulators &a)
-        : acc(a), cur(nullptr), lo(make_float4(0.0f, 0.0f, 0.0f, 0.0f)), hi(lo)
+    __device__ __forceinline__ explicit CellScatter(const CellAccumulators &a) : acc(a), cur(nullptr) { clear(); }
+    __device__ __forceinline__ void clear()
     {
+        lo[0] = lo[1] = hi[0] = hi[1] = make_float2(0.0f, 0.0f);
     }
     __device__ __forceinline__ void flush()
     {
         if (!cur) return;
-        atomicAdd(cur, lo);
-        atomicAdd(cur + 1, hi);
+        atomicAdd(cur, make_float4(lo[0].x, lo[0].y, lo[1].x, lo[1].y));
+        atomicAdd(cur + 1, make_float4(hi[0].x, hi[0].y, hi[1].x, hi[1].y));
     }
     __device__ __forceinline__ void add(float x, float y, float z, float val)
     {
-        const FloorFrac fx = floor_frac(x), fy = floor_frac(y), fz = floor_frac(z);
-        if (CHECK && ((unsigned)(fx.i + 1) > (unsigned)(acc.X + 1) || (unsigned)(fy.i + 1) > (unsigned)(acc.Y + 1) ||
+        // x and y, and the weights of each (x0, x1) pair, on the packed FP32
+        // instructions
+        constexpr float MAGIC = 12582912.0f;  // floor_frac's
+        const float2 p = make_float2(x, y), fl = __fadd2_rd(p, make_float2(MAGIC, MAGIC));
+        const float2 f = __ffma2_rn(__fadd2_rn(fl, make_float2(-MAGIC, -MAGIC)), make_float2(-1.0f, -1.0f), p);
+        const int ix = __float_as_int(fl.x) - FLOOR_BIAS, iy = __float_as_int(fl.y) - FLOOR_BIAS;
+        const FloorFrac fz = floor_frac(z);
+        if (CHECK && ((unsigned)(ix + 1) > (unsigned)(acc.X + 1) || (unsigned)(iy + 1) > (unsigned)(acc.Y + 1) ||
                       (unsigned)(fz.i + 1) > (unsigned)(acc.Z + 1)))
             return;
-        float4 *c = acc.cell(fx.i, fy.i, fz.i);
+        float4 *c = acc.cell(ix, iy, fz.i);
         if (c != cur) {
             flush();
             cur = c;
-            lo = hi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            clear();
         }
         // weights of lerp_ref(a, b, t) = a (1 - t) + b t
-        const float h = val * fz.f, l = val * (1.0f - fz.f);
-        const float ty0 = 1.0f - fy.f, tx0 = 1.0f - fx.f;
-        const float w00 = ty0 * tx0, w10 = ty0 * fx.f, w01 = fy.f * tx0, w11 = fy.f * fx.f;
-        lo.x = fmaf(l, w00, lo.x), lo.y = fmaf(l, w10, lo.y), lo.z = fmaf(l, w01, lo.z), lo.w = fmaf(l, w11, lo.w);
-        hi.x = fmaf(h, w00, hi.x), hi.y = fmaf(h, w10, hi.y), hi.z = fmaf(h, w01, hi.z), hi.w = fmaf(h, w11, hi.w);
+        const float h = val * fz.f, l = val * (1.0f - fz.f), ty0 = 1.0f - f.y;
+        const float2 wx = make_float2(1.0f - f.x, f.x);
+        const float2 w0 = __fmul2_rn(make_float2(ty0, ty0), wx), w1 = __fmul2_rn(make_float2(f.y, f.y), wx);
+        lo[0] = __ffma2_rn(make_float2(l, l), w0, lo[0]), lo[1] = __ffma2_rn(make_float2(l, l), w1, lo[1]);
+        hi[0] = __ffma2_rn(make_float2(h, h), w0, hi[0]), hi[1] = __ffma2_rn(make_float2(h, h), w1, hi[1]);
     }
 };
 
