@@ -207,6 +207,13 @@ PYRONN_API int pyronn_cone_projection3d(const void *volume, void *sinogram, int 
  * per lerp, the same results).  A workspace
  * of the per-view part alone -- this size with batch = 0 -- is accepted: the
  * call then stages the sinogram itself. */
+/* The forward's workspace with room for a second batch element's copies: given
+ * this size, elements that share their geometry (geom_batch 1) are projected two
+ * at a time, their rays' set-up and sample positions computed once.  Equal to
+ * the query above where that does not apply. */
+PYRONN_API size_t pyronn_cone_projection3d_batched_workspace_size(int batch, int vol_z, int vol_y, int vol_x,
+                                                                  int n_proj, int det_h, int det_w, int in_dtype,
+                                                                  int hardware_interp, int geom_batch);
 PYRONN_API size_t pyronn_cone_backprojection3d_workspace_size(int batch, int n_proj, int det_h, int det_w, int vol_z,
                                                               int vol_y, int vol_x, int in_dtype,
                                                               int hardware_interp, int geom_batch);

@@ -316,6 +316,17 @@ size_t pyronn_cone_projection3d_workspace_size(int batch, int vol_z, int vol_y, 
     return n;
 }
 
+size_t pyronn_cone_projection3d_batched_workspace_size(int batch, int vol_z, int vol_y, int vol_x, int n_proj,
+                                                       int det_h, int det_w, int in_dtype, int hardware_interp,
+                                                       int geom_batch)
+{
+    const size_t one = pyronn_cone_projection3d_workspace_size(batch, vol_z, vol_y, vol_x, n_proj, det_h, det_w,
+                                                               in_dtype, hardware_interp, geom_batch);
+    const Dims3D d{batch, vol_z, vol_y, vol_x, n_proj, det_h, det_w, geom_batch};
+    if (one == 0 || batch < 2 || geom_batch != 1 || hardware_interp || !cone_fp_padded_supported(d, in_dtype)) return one;
+    return one + align_up(cone_fp_padded_scratch_bytes(vol_z, vol_y, vol_x, in_dtype), 256);
+}
+
 size_t pyronn_cone_backprojection3d_workspace_size(int batch, int n_proj, int det_h, int det_w, int vol_z, int vol_y,
                                                    int vol_x, int in_dtype, int hardware_interp, int geom_batch)
 {
@@ -373,8 +384,11 @@ int pyronn_cone_projection3d(const void *volume, void *sinogram, int in_dtype, i
         if (cone_fp_padded_supported(d, in_dtype)) {
             void *scratch = (char *)workspace + WS_HEADER +
                             align_up((size_t)geom_batch * n_proj * sizeof(ConeFpView), 256);
+            const bool pairs = workspace_bytes >= pyronn_cone_projection3d_batched_workspace_size(
+                                                      batch, vol_z, vol_y, vol_x, n_proj, det_h, det_w, in_dtype,
+                                                      hardware_interp, geom_batch);
             e = launch_cone_fp_padded(volume, sinogram, in_dtype, out_dtype, d, views, step_size, volume_spacing,
-                                      scratch, (unsigned *)workspace, s);
+                                      scratch, pairs, (unsigned *)workspace, s);
         } else {
             e = launch_cone_fp(volume, sinogram, in_dtype, out_dtype, d, -1, views, step_size, volume_spacing, 0, s);
         }

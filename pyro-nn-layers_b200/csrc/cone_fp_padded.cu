@@ -442,16 +442,37 @@ struct CellSampler {
         base = (unsigned long long)cells + sizeof(C) * (origin - cell_index_bias(s_x, s_y, Z2));
     }
 
+    // at the address `base` + index: this copy's, or another's of the same shape
+    __device__ __forceinline__ float at(unsigned long long from, unsigned t, float tz, float ty, float tx) const
+    {
+        const C *c = (const C *)(from + (unsigned long long)t * sizeof(C));
+        // the reference's order: lerp in z, then y, then x
+        if constexpr (PACKED)
+            return Cell<T>::trilinear_packed(c, tz, ty, tx);
+        else
+            return Cell<T>::trilinear(c, tz, ty, tx);
+    }
+
     __device__ __forceinline__ float operator()(float x, float y, float z) const
     {
         const FloorFrac fx = floor_frac(x), fy = floor_frac(y), fz = Z2 ? floor_frac_2z(z) : floor_frac(z);
         const unsigned t = (unsigned)fx.bits * s_x + (unsigned)fy.bits * s_y + (unsigned)fz.bits;
-        const C *c = (const C *)(base + (unsigned long long)t * sizeof(C));
-        // the reference's order: lerp in z, then y, then x
-        if constexpr (PACKED)
-            return Cell<T>::trilinear_packed(c, fz.f, fy.f, fx.f);
-        else
-            return Cell<T>::trilinear(c, fz.f, fy.f, fx.f);
+        return at(base, t, fz.f, fy.f, fx.f);
+    }
+};
+
+// The same position in NS copies, `stride` bytes apart.
+template <typename T, bool PACKED, int NS>
+struct MultiCellSampler {
+    CellSampler<T, PACKED> s;
+    unsigned long long stride;
+    __device__ __forceinline__ void operator()(float x, float y, float z, float (&v)[NS]) const
+    {
+        const FloorFrac fx = floor_frac(x), fy = floor_frac(y),
+                        fz = CellSampler<T, PACKED>::Z2 ? floor_frac_2z(z) : floor_frac(z);
+        const unsigned t = (unsigned)fx.bits * s.s_x + (unsigned)fy.bits * s.s_y + (unsigned)fz.bits;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) v[k] = s.at(s.base + k * stride, t, fz.f, fy.f, fx.f);
     }
 };
 
@@ -489,22 +510,59 @@ __device__ __forceinline__ float march_cells(const ConeRay &ray, float step, boo
                     : march_x2(r, step, ClampedCellSampler<T, PACKED>{s, xmax, ymax, zlo, zmax});
 }
 
+// The march of one z-mode ray over the cell copies of NS volumes, `stride`
+// bytes apart.
+template <typename T, bool PACKED, int NS>
+__device__ __forceinline__ void march_cells_multi(const ConeRay &ray, float step, bool inside,
+                                                  const typename Cell<T>::type *cells, size_t stride, int Z, int s_x,
+                                                  float xmax, float ymax, float zmax, float (&pixel)[NS])
+{
+    if constexpr (NS == 1) {
+        pixel[0] = march_cells<T, PACKED>(ray, step, inside, cells, Z, s_x, xmax, ymax, zmax);
+    } else {
+        const int n = inside ? exact_sample_count(ray, step) : -1;
+        if (n > 0) {
+            ConeRay r = ray;
+            if (CellSampler<T, PACKED>::Z2) r.dz *= 2.0f, r.oz *= 2.0f;
+            const MultiCellSampler<T, PACKED, NS> s{CellSampler<T, PACKED>(cells, Z + Cell<T>::PLANES, s_x), stride};
+            constexpr int U = sizeof(T) == 4 ? 2 : 4;  // samples per iteration, in 64 registers
+            march_counted_multi<U, NS>(r, n, step, s, pixel);
+        } else {
+#pragma unroll 1
+            for (int k = 0; k < NS; ++k) {
+                const float v = march_cells<T, PACKED>(
+                    ray, step, inside, (const typename Cell<T>::type *)((const char *)cells + k * stride), Z, s_x, xmax,
+                    ymax, zmax);
+                pixel[0] = k == 0 ? v : pixel[0];
+                pixel[NS - 1] = k == NS - 1 ? v : pixel[NS - 1];
+            }
+        }
+    }
+}
+
 // Grid: one dimension, ray_block_count blocks in ray_block order (four
 // blocks of 256 threads per 32 x 32 ray tile, neighbouring views of a tile
 // consecutive, cone_ray.cuh).  z mode: a warp is 32 consecutive v at one u, and the
 // block's 8 x 32 results go through shared memory so the sinogram rows are
 // written 8 pixels at a time; xy mode: a warp is 32 consecutive u.
-template <typename T, typename Tout>
+// NS = 2: batch elements b and b + 1, which share their geometry, their copies
+// `stride` bytes apart; a ray's set-up and sample positions (about 22 of the 38
+// instructions of a sample at 128^3) are computed once.  Four volumes of 128^3,
+// 180 views of 256^2: FP32 7.22 -> 6.34 ms (the L1's lines bound it then), FP16
+// 5.98 -> 4.34; two of 181 x 203 x 219, 271 views of 287 x 347, BF16 11.8 -> 8.2.
+// (More samples per iteration, or 3 blocks per SM: 1 to 5 % slower.)
+template <typename T, typename Tout, int NS>
 // (4 blocks per SM: 64 registers hold the counted loop without spills, and
 // 32 resident warps hide the cell loads better than 24 with 80 registers)
 __global__ void __launch_bounds__(PB_X *PB_Y, 4)
     cone_fp_padded_kernel(const T *__restrict__ xfast, const T *__restrict__ yfast,
-                          const typename Cell<T>::type *__restrict__ cells, Tout *__restrict__ sino,
+                          const typename Cell<T>::type *__restrict__ cells, size_t stride, Tout *__restrict__ sino,
                           const ConeFpView *__restrict__ views, const float *__restrict__ step_ptr,
                           const float *__restrict__ spacing_ptr, int X, int Y, int Z, int cell_sx, int W, int H,
                           int n_proj, int geom_batch, int b, const unsigned *__restrict__ flags)
 {
-    __shared__ float out_tile[PB_Y][PB_X + 1];
+    static_assert(NS <= 2, "one or two volumes");
+    __shared__ float out_tile[NS][PB_Y][PB_X + 1];
     const RayBlock rb = ray_block(blockIdx.x, W, H, n_proj);
     const int p = rb.p, sub = rb.sub, tile_u = rb.tile_u, tile_v = rb.tile_v;
     const int g = geom_batch == 1 ? 0 : b;
@@ -522,7 +580,9 @@ __global__ void __launch_bounds__(PB_X *PB_Y, 4)
     const float step = step_ptr[g];
     // 16-bit cells take the packed lerps unless the input's range forbids them
     const bool packed = sizeof(T) == 2 && !flags[FLAG_WIDE];
-    float pixel = 0.0f;
+    float pixel[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) pixel[k] = 0.0f;
     if (live && in_footprint(view, u, v)) {
         const ConeRay ray = cone_ray_setup(view, u, v, X, Y, Z, 0.0, step, spacing_ptr[g * 3 + 2],
                                            spacing_ptr[g * 3 + 1], spacing_ptr[g * 3 + 0]);
@@ -531,36 +591,53 @@ __global__ void __launch_bounds__(PB_X *PB_Y, 4)
         const int Xp = X + 3, Yp = Y + 3;
         if (zmode) {
             if (packed)
-                pixel = march_cells<T, sizeof(T) == 2>(ray, step, inside, cells, Z, cell_sx, xmax, ymax, zmax);
+                march_cells_multi<T, sizeof(T) == 2, NS>(ray, step, inside, cells, stride, Z, cell_sx, xmax, ymax,
+                                                         zmax, pixel);
             else
-                pixel = march_cells<T, false>(ray, step, inside, cells, Z, cell_sx, xmax, ymax, zmax);
+                march_cells_multi<T, false, NS>(ray, step, inside, cells, stride, Z, cell_sx, xmax, ymax, zmax, pixel);
         } else {
             // rays mostly along x -> y-fastest copy
             const double cr0 = view.inv_ar[2] + 0.5 * (W - 1) * view.inv_ar[0] + 0.5 * (H - 1) * view.inv_ar[1];
             const double cr1 = view.inv_ar[5] + 0.5 * (W - 1) * view.inv_ar[3] + 0.5 * (H - 1) * view.inv_ar[4];
             const int s_slice = Xp * Yp;
-            if (fabs(cr0) > fabs(cr1)) {
-                const PaddedSampler<T, true> s{yfast + s_slice + Yp + 1, Yp, s_slice};
-                pixel = inside ? march_x2(ray, step, s)
-                               : march_x2(ray, step, ClampedSampler<T, true>{s, xmax, ymax, zmax});
-            } else {
-                const PaddedSampler<T, false> s{xfast + s_slice + Xp + 1, Xp, s_slice};
-                pixel = inside ? march_x2(ray, step, s)
-                               : march_x2(ray, step, ClampedSampler<T, false>{s, xmax, ymax, zmax});
+            const bool fast_y = fabs(cr0) > fabs(cr1);
+#pragma unroll 1
+            for (int k = 0; k < NS; ++k) {
+                float value;
+                if (fast_y) {
+                    const T *copy = (const T *)((const char *)yfast + k * stride);
+                    const PaddedSampler<T, true> s{copy + s_slice + Yp + 1, Yp, s_slice};
+                    value = inside ? march_x2(ray, step, s)
+                                   : march_x2(ray, step, ClampedSampler<T, true>{s, xmax, ymax, zmax});
+                } else {
+                    const T *copy = (const T *)((const char *)xfast + k * stride);
+                    const PaddedSampler<T, false> s{copy + s_slice + Xp + 1, Xp, s_slice};
+                    value = inside ? march_x2(ray, step, s)
+                                   : march_x2(ray, step, ClampedSampler<T, false>{s, xmax, ymax, zmax});
+                }
+                pixel[0] = k == 0 ? value : pixel[0];
+                pixel[NS - 1] = k == NS - 1 ? value : pixel[NS - 1];
             }
         }
     }
     Tout *out = sino + ((size_t)b * n_proj + p) * H * (size_t)W;
+    const size_t sino_stride = (size_t)n_proj * H * W;
     if (!zmode) {
-        if (live) store_from_float(out + (size_t)v * W + u, pixel);
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+            if (live) store_from_float(out + k * sino_stride + (size_t)v * W + u, pixel[k]);
         return;
     }
     // z mode: transpose the 8 (u) x 32 (v) results so each row is written as 8 pixels
-    out_tile[threadIdx.y][threadIdx.x] = pixel;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) out_tile[k][threadIdx.y][threadIdx.x] = pixel[k];
     __syncthreads();
     const int t = threadIdx.y * PB_X + threadIdx.x;
     const int ov = tile_v * 32 + t / PB_Y, ou = tile_u * 32 + sub * PB_Y + t % PB_Y;
-    if (ov < H && ou < W) store_from_float(out + (size_t)ov * W + ou, out_tile[t % PB_Y][t / PB_Y]);
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+        if (ov < H && ou < W)
+            store_from_float(out + k * sino_stride + (size_t)ov * W + ou, out_tile[k][t % PB_Y][t / PB_Y]);
 }
 
 size_t section_bytes(size_t n)
@@ -596,17 +673,17 @@ long long cell_x_pitch(int vol_x, int vol_y, int vol_z, size_t elem)
 
 template <typename Tin, typename Tout>
 cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, const ConeFpView *views,
-                         const float *step, const float *spacing, void *scratch, unsigned *flags, cudaStream_t stream)
+                         const float *step, const float *spacing, void *scratch, bool pairs, unsigned *flags,
+                         cudaStream_t stream)
 {
     using CellT = typename Cell<Tin>::type;
     const size_t Xp = d.vol_x + 3, Yp = d.vol_y + 3, Zp = d.vol_z + 3;
     const size_t Xc = d.vol_x + 2, Yc = d.vol_y + 2, Zc = d.vol_z + Cell<Tin>::PLANES;
     const long long cell_sx = cell_x_pitch(d.vol_x, d.vol_y, d.vol_z, sizeof(Tin));
     if (cell_sx <= 0) return cudaErrorInvalidValue;
-    char *base = (char *)scratch;
-    Tin *xfast = (Tin *)base;
-    Tin *yfast = (Tin *)(base + section_bytes(Xp * Yp * Zp * sizeof(Tin)));
-    CellT *cells = (CellT *)(base + 2 * section_bytes(Xp * Yp * Zp * sizeof(Tin)));
+    const size_t stride = section_bytes(cone_fp_padded_scratch_bytes(d.vol_z, d.vol_y, d.vol_x,
+                                                                     sizeof(Tin) == 4 ? PYRONN_FLOAT32 : PYRONN_FLOAT16));
+    const size_t padded = section_bytes(Xp * Yp * Zp * sizeof(Tin));
     const int nviews = d.geom_batch * d.n_proj;
     classify_views_kernel<<<(nviews + 127) / 128, 128, 0, stream>>>(views, nviews, flags);
     const dim3 pblock(PAD_TILE, 8);
@@ -616,22 +693,37 @@ cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, co
                      (unsigned)((Zc + PAD_TILE - 1) / PAD_TILE));
     const dim3 block(PB_X, PB_Y);
     const unsigned grid = ray_block_count(d.det_w, d.det_h, d.n_proj);
-    for (int b = 0; b < d.batch; ++b) {
-        const Tin *src = (const Tin *)volume + (size_t)b * d.vol_z * d.vol_y * d.vol_x;
-        pad_volume_kernel<Tin><<<pgrid, pblock, 0, stream>>>(src, xfast, yfast, d.vol_x, d.vol_y, d.vol_z, flags);
+    const size_t n = (size_t)d.vol_z * d.vol_y * d.vol_x;
+    for (int b = 0; b < d.batch;) {
+        const int ns = pairs && d.geom_batch == 1 && b + 1 < d.batch ? 2 : 1;
+        auto copies = [&](int k, Tin *&xfast, Tin *&yfast, CellT *&cells) {
+            char *base = (char *)scratch + k * stride;
+            xfast = (Tin *)base, yfast = (Tin *)(base + padded), cells = (CellT *)(base + 2 * padded);
+        };
+        Tin *xfast, *yfast;
+        CellT *cells;
         if constexpr (sizeof(Tin) == 2) {
-            const size_t n = (size_t)d.vol_z * d.vol_y * d.vol_x;
-            const unsigned wgrid = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 8);
-            detect_wide_kernel<Tin><<<wgrid, 256, 0, stream>>>(src, n, flags);
+            // the cells' form depends on the range of all the launch's volumes
+            const unsigned wgrid = (unsigned)std::min<size_t>((ns * n + 255) / 256, 148 * 8);
+            detect_wide_kernel<Tin><<<wgrid, 256, 0, stream>>>((const Tin *)volume + b * n, ns * n, flags);
         }
-        pad_cells_kernel<Tin><<<cgrid, pblock, 0, stream>>>(src, cells, d.vol_x, d.vol_y, d.vol_z, (int)cell_sx,
-                                                             flags);
-        cone_fp_padded_kernel<Tin, Tout><<<grid, block, 0, stream>>>(xfast, yfast, cells, (Tout *)sinogram, views,
-                                                                     step, spacing, d.vol_x, d.vol_y, d.vol_z,
-                                                                     (int)cell_sx, d.det_w, d.det_h, d.n_proj,
-                                                                     d.geom_batch, b, flags);
+        for (int k = 0; k < ns; ++k) {
+            const Tin *src = (const Tin *)volume + (b + k) * n;
+            copies(k, xfast, yfast, cells);
+            pad_volume_kernel<Tin><<<pgrid, pblock, 0, stream>>>(src, xfast, yfast, d.vol_x, d.vol_y, d.vol_z, flags);
+            pad_cells_kernel<Tin><<<cgrid, pblock, 0, stream>>>(src, cells, d.vol_x, d.vol_y, d.vol_z, (int)cell_sx,
+                                                                 flags);
+        }
+        copies(0, xfast, yfast, cells);
+        auto launch = [&](auto kernel) {
+            kernel<<<grid, block, 0, stream>>>(xfast, yfast, cells, stride, (Tout *)sinogram, views, step, spacing,
+                                               d.vol_x, d.vol_y, d.vol_z, (int)cell_sx, d.det_w, d.det_h, d.n_proj,
+                                               d.geom_batch, b, flags);
+        };
+        ns == 2 ? launch(cone_fp_padded_kernel<Tin, Tout, 2>) : launch(cone_fp_padded_kernel<Tin, Tout, 1>);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
+        b += ns;
     }
     return cudaSuccess;
 }
@@ -659,12 +751,13 @@ bool cone_fp_padded_supported(const Dims3D &d, int in_dtype)
 
 cudaError_t launch_cone_fp_padded(const void *volume, void *sinogram, int in_dtype, int out_dtype, const Dims3D &d,
                                   const ConeFpView *views, const float *step, const float *spacing, void *scratch,
-                                  unsigned *flags, cudaStream_t stream)
+                                  bool pairs, unsigned *flags, cudaStream_t stream)
 {
     return dispatch_dtypes(in_dtype, out_dtype, [&](auto tin, auto tout) {
         using Tin = typename decltype(tin)::type;
         using Tout = typename decltype(tout)::type;
-        return launch_typed<Tin, Tout>(volume, sinogram, d, views, step, spacing, scratch, flags, stream);
+        return launch_typed<Tin, Tout>(volume, sinogram, d, views, step, spacing, scratch, pairs, flags,
+                                       stream);
     });
 }
 

@@ -277,6 +277,53 @@ __device__ __forceinline__ float march_counted(const ConeRay &ray, int n, float 
     return pixel * ray.mm_scale;
 }
 
+// march_counted for NS volumes sampled at the same positions:
+// sample(x, y, z, v) fills v[0 .. NS).
+template <int U, int NS, typename F>
+__device__ __forceinline__ void march_counted_multi(const ConeRay &ray, int n, float step, const F &sample,
+                                                    float (&pixel)[NS])
+{
+    float a = ray.a, last[NS];
+    sample(fmaf(a, ray.dx, ray.ox), fmaf(a, ray.dy, ray.oy), fmaf(a, ray.dz, ray.oz), last);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) pixel[s] = 0.5f * last[s];
+    a += step;
+    int k = 1;
+    for (; k + U - 1 < n; k += U) {
+        float v[U][NS];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            sample(fmaf(a, ray.dx, ray.ox), fmaf(a, ray.dy, ray.oy), fmaf(a, ray.dz, ray.oz), v[j]);
+            a += step;
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+#pragma unroll
+            for (int j = 0; j < U; ++j) pixel[s] += v[j][s];
+            last[s] = v[U - 1][s];
+        }
+    }
+    for (; k < n; ++k) {
+        sample(fmaf(a, ray.dx, ray.ox), fmaf(a, ray.dy, ray.oy), fmaf(a, ray.dz, ray.oz), last);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) pixel[s] += last[s];
+        a += step;
+    }
+    float end[NS];
+    sample(fmaf(ray.am, ray.dx, ray.ox), fmaf(ray.am, ray.dy, ray.oy), fmaf(ray.am, ray.dz, ray.oz), end);
+    const float last_step = ray.am - (a - step);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        pixel[s] *= step;
+        if (pixel[s] > 0.0f) {
+            pixel[s] -= 0.5f * step * last[s];
+            pixel[s] += 0.5f * last_step * last[s];
+            pixel[s] += 0.5f * last_step * end[s];
+        }
+        pixel[s] *= ray.mm_scale;
+    }
+}
+
 // Number of samples of the march when its float alpha sequence is exact:
 // step a multiple of ulp(a0) and every alpha up to the one after the last
 // sample below the next power of two above a0, so each a += step adds

@@ -48,6 +48,7 @@ PROTOTYPES = {
         _I, [_P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _P, _SZ, _P]),
     "pyronn_fan_backprojection2d": (_I, [_P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _I, _P]),
     "pyronn_cone_projection3d_workspace_size": (_SZ, [_I] * 10),
+    "pyronn_cone_projection3d_batched_workspace_size": (_SZ, [_I] * 10),
     "pyronn_cone_projection3d": (
         _I, [_P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _I, _P, _SZ, _P]),
     "pyronn_cone_backprojection3d_workspace_size": (_SZ, [_I] * 10),

@@ -411,9 +411,10 @@ def _run_cone(forward: bool, x: torch.Tensor, out_dims, geo: GeometryCone, hardw
         ws_args = dims + [storage_code(x.dtype), int(bool(hardware_interp)), geo.g]
     ws_bytes = _capi.workspace_size(fn, *ws_args)
     if workspace is None or workspace.numel() < ws_bytes:
-        # a backprojection's query without a batch is its per-view part alone
-        least = None if forward else lambda: _capi.workspace_size(fn, 0, *ws_args[1:])
-        workspace = _workspace(ws_bytes, dev, least)
+        if forward:  # room for two elements' copies, else for one's
+            workspace = _workspace(_capi.workspace_size(fn + "_batched", *ws_args), dev, lambda: ws_bytes)
+        else:  # the query without a batch is the per-view part alone
+            workspace = _workspace(ws_bytes, dev, lambda: _capi.workspace_size(fn, 0, *ws_args[1:]))
     with _on_device(dev):
         _capi.call(fn, x.data_ptr(), out.data_ptr(), storage_code(x.dtype), storage_code(od),
                    int(bool(hardware_interp)), *dims, *geo.pointers(), geo.g, workspace.data_ptr(),

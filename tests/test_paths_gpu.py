@@ -10,7 +10,7 @@ import torch
 
 import oracle
 import pyronn_layers as pl
-from pyronn_layers import _capi, fbp, geometry
+from pyronn_layers import _capi, fbp, geometry, phantoms
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -251,3 +251,44 @@ def test_filter_keeps_rows_apart(cuda):
                                                                    clean[0, 0, r].cpu().numpy()) < 1e-6
     assert torch.isnan(out[0, 0, 1]).all() and torch.isnan(out[0, 0, 4]).all()
     assert (out[0, 0, 6] == 0).all()
+
+
+# ---------------------------------------------------- cone forward, batches
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,tilt", [(2, 0.0), (3, 0.0), (2, 0.5 * np.pi), (3, 0.4)])
+def test_cone_forward_pairs_are_bit_exact(cuda, batch, tilt, dtype):
+    """Two elements per launch (given the batched workspace) take the same
+    samples in the same order as one at a time: the same bits, in every view
+    mode, for an odd element left over, and for rays on the clamped path."""
+    geo = geometry.ConeBeam3D((21, 26, 30), (1.0, 0.9, 1.1), (33, 41), (1.2, 1.3), 9, 60.0, 110.0, step_size=0.5)
+    args = (geo.volume_origin, geo.volume_spacing, _tilted(geo, tilt), geo.step_size, 1.0)
+    x = t(noise(41, (batch,) + geo.volume_shape), cuda, dtype)
+    g = pl.ops.GeometryCone(batch, cuda, *args, geo.detector_shape[0])
+    code = pl.ops.storage_code(dtype)
+    name, dims = "pyronn_cone_projection3d", (batch, *geo.volume_shape, *geo.detector_shape)
+    outs = []
+    for query in (name, name + "_batched"):
+        n = _capi.workspace_size(query, *dims, code, 0, g.g)
+        ws = torch.empty(n, dtype=torch.uint8, device=cuda)
+        out = torch.full((batch,) + geo.detector_shape, 7.0, device=cuda)
+        _capi.call(name, x.data_ptr(), out.data_ptr(), code, 0, 0, *dims, *g.pointers(), g.g, ws.data_ptr(), n,
+                   torch.cuda.current_stream().cuda_stream)
+        outs.append((n, out))
+    assert outs[1][0] > outs[0][0]
+    assert torch.equal(outs[0][1], outs[1][1]) and bool((outs[1][1] != 0).any())
+
+
+def test_cone_forward_pair_of_wide_range(cuda):
+    """FP16 values beyond the packed lerps' range in the second element of a
+    pair: both take the FP32 lerps (test_cone_projection_wide_fp16_range's
+    tolerance)."""
+    geo = geometry.ConeBeam3D((21, 26, 30), (1.0, 0.9, 1.1), (33, 41), (1.2, 1.3), 5, 60.0, 110.0, step_size=0.5)
+    vol = np.stack([phantoms.ellipsoid_phantom_3d(geo.volume_shape, geo.volume_spacing, seed=s, n=6)[0] for s in (1, 2)])
+    vol[1] *= 60000.0 / vol[1].max()
+    x = t(vol, cuda, torch.float16)
+    out = pl.cone_projection3d(x, geo.detector_shape, *geo.args(), out_dtype=torch.float32)
+    ref = oracle.cone_projection3d(x.float().cpu().numpy(), geo.detector_shape, *geo.args())
+    for b in range(2):
+        assert rel_l2(out[b].cpu().numpy(), ref[b]) < 2e-5
