@@ -32,13 +32,13 @@ def noise(seed, shape):
     (1, 9, 40),      # ray segments (one band of columns per thread)
     (1, 97, 3100),   # one thread per ray, one slice (above the segments' limit)
     (2, 97, 780),    # two slices per thread
-    (3, 83, 610),    # two slices per thread, the last pair overlapping
+    (3, 83, 610),    # three slices per thread
     (4, 83, 460),    # four slices per thread
-    (5, 61, 500),    # four per thread, the last group overlapping
+    (5, 61, 500),    # three per thread, the last group overlapping
+    (7, 61, 400),    # four per thread, the last group overlapping
 ])
 def test_2d_forward_walks(cuda, batch, views, width, fan):
-    """Every walk of the 2D forward (segments; one, two and four slices per
-    thread) against the oracle, and without the workspace the same bits."""
+    """Every walk of the 2D forward (segments; one to four slices per thread) against the oracle, and without the workspace the same bits."""
     shape, sp, ds = (23, 37), (0.8, 1.0), 60.0 / width
     if fan:
         geo = geometry.FanBeam2D(shape, sp, width, ds, views, 60.0, 90.0)
@@ -90,12 +90,13 @@ def test_2d_forward_source_inside(cuda):
 @pytest.mark.parametrize("batch,shape,views,width,dtype", [
     (1, (33, 65), 70, 90, torch.float32),       # one slice, view groups
     (2, (31, 33), 257, 60, torch.bfloat16),     # two slices per thread; two view chunks
-    (3, (40, 37), 33, 91, torch.float32),       # two per thread, the last pair overlapping
-    (5, (40, 37), 33, 30, torch.float16),       # four per thread, overlapping; pixels off the detector
+    (3, (40, 37), 33, 91, torch.float32),       # three per thread
+    (5, (40, 37), 33, 30, torch.float16),       # three per thread, overlapping; pixels off the detector
+    (7, (40, 37), 33, 91, torch.bfloat16),      # four per thread, overlapping
 ])
 def test_2d_backprojection_walks(cuda, batch, shape, views, width, dtype, fan):
-    """The splits of the 2D backprojection (view groups; one, two and four
-    slices per thread; blocks wholly inside the detector rows and blocks that
+    """The splits of the 2D backprojection (view groups; one to four slices per
+    thread; blocks wholly inside the detector rows and blocks that
     need tap flags) against the oracle."""
     if fan:
         geo = geometry.FanBeam2D(shape, (0.8, 1.0), width, 1.1, views, 900.0, 1300.0)
@@ -110,7 +111,7 @@ def test_2d_backprojection_walks(cuda, batch, shape, views, width, dtype, fan):
 
 
 @pytest.mark.parametrize("fan", [False, True])
-@pytest.mark.parametrize("batch,shape,dtype", [(6, (900, 800), torch.float32), (9, (960, 940), torch.float16)])
+@pytest.mark.parametrize("batch,shape,dtype", [(7, (900, 800), torch.float32), (9, (960, 940), torch.float16)])
 def test_2d_backprojection_shared_slices(cuda, batch, shape, dtype, fan):
     """Launches without view groups: four and eight slices per thread (the last
     group overlapping) give each slice the bits of a call of its own."""
