@@ -330,11 +330,11 @@ PYRONN_API int pyronn_circular_ray_vectors_2d(float *ray_vectors, int n_proj, do
  * of the weight-then-filter operator, the kernel being symmetric).  FDK =
  * this, then pyronn_cone_backprojection3d with projection_multiplier
  * SID * SDD * pi / n_proj (full circle).  projections and filtered may be
- * the same buffer.  det_w <= PYRONN_FDK_MAX_WIDTH.  Distinct buffers with
- * det_w a multiple of 4 up to 2048 (16-byte aligned) run on the tensor cores
- * (the Toeplitz product in 3xTF32, FP32-accurate: within a few 1e-6 relative
- * of the CUDA-core kernel); in-place calls and other widths on the CUDA
- * cores (FP32 FMAs).
+ * the same buffer (of one storage type).  det_w <= PYRONN_FDK_MAX_WIDTH.  Rows
+ * of up to 2048 pixels go through FP32 Fourier transforms of the row
+ * differences (about 1.5e-7 relative of the exact filter), wider ones are
+ * direct FP32 sums.  A row holding infinities or NaNs comes back as NaNs;
+ * others are not affected by it.
  * ------------------------------------------------------------------------- */
 #define PYRONN_FILTER_RAM_LAK 0
 #define PYRONN_FILTER_SHEPP_LOGAN 1
@@ -345,10 +345,8 @@ PYRONN_API int pyronn_fdk_filter(const void *projections, void *filtered, int in
                                  double det_spacing_u, double principal_v, double principal_u, int filter,
                                  int weight_output, void *stream);
 
-/* Reads and clears the device error flag of the tensor-core filter on the
- * current device: PYRONN_DEVICE_ERROR_WAIT_TIMEOUT if a bounded wait of any
- * pyronn_fdk_filter call since the last read gave up (that call's rows of the
- * affected tile were not written), else PYRONN_DEVICE_ERROR_NONE.
+/* The device error flag of pyronn_fdk_filter calls on the current device: its
+ * kernels wait on nothing that could fail, so PYRONN_DEVICE_ERROR_NONE.
  * Synchronises the stream. */
 PYRONN_API int pyronn_fdk_error(void *stream, int *device_error);
 

@@ -91,8 +91,8 @@ class PyronnDeviceError(RuntimeError):
 
     def __init__(self, flags, what="device"):
         self.flags = flags
-        super().__init__("%s error flags 0x%x: a bounded wait for an asynchronous copy or tensor-core "
-                         "operation gave up; the affected output was not written" % (what, flags))
+        super().__init__("%s error flags 0x%x: a bounded wait for an asynchronous copy "
+                         "gave up; the affected output was not written" % (what, flags))
 
 
 def _status_name(status):

@@ -19,8 +19,8 @@ mirrors ``REGISTER_OP("ConeProjection3D")`` (cc/ops/cone_projector_3D_OPKernel.c
   vice versa (the pairing the PYRO-NN package registers for these ops); the
   geometry inputs get no gradient.
 * Errors raise :class:`~pyronn_layers._capi.PyronnError` (the reference exits
-  the process or ignores CUDA errors).  Kernels with bounded device-side waits
-  (the TMA-staged cone backprojector, the tensor-core FDK filter) report a
+  the process or ignores CUDA errors).  The kernel with bounded device-side
+  waits (the TMA-staged cone backprojector) reports a
   wait that gave up through a device flag after the call has returned: the
   ops fold those flags into a per-device word on the stream, without
   synchronising, and :func:`check_device_errors` (or ``device_errors``) reads
@@ -200,8 +200,8 @@ def note_workspace_error(workspace: torch.Tensor, device) -> None:
 
 def device_errors(device=None, clear: bool = True) -> int:
     """Synchronises the device and returns the OR of the device error flags
-    raised since the last call (pyronn_layers ops' workspaces and the
-    tensor-core FDK filter's word): 0 when every bounded wait completed,
+    raised since the last call (pyronn_layers ops' workspaces and the FDK
+    filter's word): 0 when every bounded wait completed,
     _capi.DEVICE_ERROR_WAIT_TIMEOUT when one gave up and its output was not
     written."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
