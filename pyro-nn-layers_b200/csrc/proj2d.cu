@@ -234,14 +234,15 @@ struct Run2D {
 // warp's loads fall on few columns, at neighbouring n.  Free-running lanes
 // spread over as many columns as lines (10 L1 cycles per load, the L1 98 %
 // busy); strict alignment (COLS = 1) idles lanes whose neighbours cross more
-// rows.  64 fan slices of 512^2, four per thread: 21.7 ms free-running, 17.0 /
-// 14.4 / 13.5 / 13.2 / 13.5 ms for COLS = 1 / 2 / 4 / 8 / 16; with one slice per
-// thread 16 is best.
+// rows.  64 fan slices of 512^2, four per thread: 21.7 ms free-running; 17.0
+// and 14.4 ms for COLS = 1 and 2 in scalar arithmetic; packed, 11.63 / 11.72 /
+// 11.93 / 12.37 / 12.84 ms for 4 / 6 / 8 / 12 / 16.  With one slice per thread 16 is
+// best, with three 8 (0.460 ms against 0.473 for 4 on 387 x 451 slices).
 template <int NS, typename Taps>
 __device__ __forceinline__ float sum_cells(const Ray2D &ray, float a, int kmax, const Taps &taps, unsigned mask,
                                            float (&acc)[NS], float &a_last)
 {
-    constexpr int COLS = NS == 1 ? 16 : 8;
+    constexpr int COLS = NS == 1 ? 16 : (NS == 4 ? 4 : 8);
 #pragma unroll
     for (int s = 0; s < NS; ++s) acc[s] = 0.0f;
     Run2D run;
