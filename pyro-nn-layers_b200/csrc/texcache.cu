@@ -65,9 +65,61 @@ __global__ void fill_layered_kernel(const T *__restrict__ src, cudaSurfaceObject
         surf2DLayeredwrite(v, surf, x * (int)sizeof(float), y, layer);
 }
 
+// Four consecutive values, widened (p aligned to four).
+__device__ __forceinline__ float4 load4(const float *p)
+{
+    return __ldg(reinterpret_cast<const float4 *>(p));
+}
+__device__ __forceinline__ float4 load4(const __half *p)
+{
+    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&q.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&q.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float4 load4(const __nv_bfloat16 *p)
+{
+    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+    return make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u), __uint_as_float(q.y << 16),
+                       __uint_as_float(q.y & 0xFFFF0000u));
+}
+
+// Rows of a multiple of four texels: four texels per thread, threads over all
+// the array's texels (the arrays of a 160^3 scan, 240 views of 320^2 in FP32: 151 us
+// in the kernels above, a texel per thread and rows that leave a part of each
+// block idle, 45 us here).
+template <typename T, bool HALF, bool LAYERED>
+__global__ void __launch_bounds__(256) fill_quads_kernel(const T *__restrict__ src, cudaSurfaceObject_t surf,
+                                                         unsigned w4, unsigned h, unsigned quads)
+{
+    const unsigned i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= quads) return;
+    const unsigned row = i / w4, x = i - row * w4;
+    const int z = (int)(row / h), y = (int)(row - (unsigned)z * h);
+    const float4 v = load4(src + (size_t)i * 4);
+    if constexpr (HALF) {
+        const ushort4 q = make_ushort4(__half_as_ushort(__float2half_rn(v.x)), __half_as_ushort(__float2half_rn(v.y)),
+                                       __half_as_ushort(__float2half_rn(v.z)), __half_as_ushort(__float2half_rn(v.w)));
+        LAYERED ? surf2DLayeredwrite(q, surf, (int)(x * sizeof(q)), y, z) : surf3Dwrite(q, surf, (int)(x * sizeof(q)), y, z);
+    } else {
+        LAYERED ? surf2DLayeredwrite(v, surf, (int)(x * sizeof(v)), y, z) : surf3Dwrite(v, surf, (int)(x * sizeof(v)), y, z);
+    }
+}
+
 template <typename T>
 cudaError_t fill_typed(CachedArray *a, const void *src, cudaStream_t stream)
 {
+    if (a->w % 4 == 0 && (uintptr_t)src % (4 * sizeof(T)) == 0) {
+        const unsigned w4 = a->w / 4, quads = w4 * (unsigned)a->h * (unsigned)a->d;  // below 2^29
+        auto launch = [&](auto kernel) {
+            kernel<<<(quads + 255) / 256, 256, 0, stream>>>((const T *)src, a->surf, w4, (unsigned)a->h, quads);
+        };
+        if (a->kind == ARRAY_VOLUME_3D)
+            a->half_texels ? launch(fill_quads_kernel<T, true, false>) : launch(fill_quads_kernel<T, false, false>);
+        else
+            a->half_texels ? launch(fill_quads_kernel<T, true, true>) : launch(fill_quads_kernel<T, false, true>);
+        return cudaGetLastError();
+    }
     // extents are bounded by the texture limits (<= 65535 in y and z)
     const dim3 block(128);
     const dim3 grid((a->w + 127) / 128, a->h, a->d);

@@ -293,3 +293,26 @@ def test_cone_forward_pair_of_wide_range(cuda):
     ref = oracle.cone_projection3d(x.float().cpu().numpy(), geo.detector_shape, *geo.args())
     for b in range(2):
         assert rel_l2(out[b].cpu().numpy(), ref[b]) < 2e-5
+
+
+# ------------------------------------------------------ texture interpolation
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("width", [20, 21, 22])
+def test_texture_fill_widths(cuda, width, dtype):
+    """Texture arrays filled four texels per thread (widths of a multiple of
+    four, aligned input) and one at a time hold the same texels: both ops of
+    a batch whose second element starts off the four-texel alignment equal a
+    call per element."""
+    geo = geometry.ConeBeam3D((5, 7, width), (1.0, 0.9, 1.1), (9, width), (1.2, 1.3), 3, 60.0, 100.0, step_size=0.5)
+    for op, shape, out_shape in ((pl.cone_projection3d, geo.volume_shape, geo.detector_shape),
+                                 (pl.cone_backprojection3d, geo.detector_shape, geo.volume_shape)):
+        n = int(np.prod(shape))
+        store = t(noise(51, (2 * n + 1,)), cuda, dtype)
+        aligned, shifted = store[:2 * n].view((2,) + shape), store[1:].view((2,) + shape)
+        for x in (aligned, shifted):
+            both = op(x, out_shape, *geo.args(), hardware_interp=True)
+            for b in range(2):
+                one = op(x[b:b + 1].clone(), out_shape, *geo.args(), hardware_interp=True)
+                assert torch.equal(one[0], both[b])
