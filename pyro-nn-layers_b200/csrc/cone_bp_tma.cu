@@ -2,8 +2,8 @@
 // tiles (software interpolation, the reference's default hardware_interp=false
 // path, cone_backprojector_3D_CudaKernel.cu.cc:84-118).
 //
-// Block = 256 threads = 32 (x) x 8 (y) voxels, each thread walks 16 voxels
-// along z: a 32 x 8 x 16 voxel tile.  Views are processed in passes of
+// Block = 256 threads = 32 (x) x 8 (y) voxels, each thread walks TB_Z voxels
+// along z (16 or 32): a 32 x 8 x TB_Z voxel tile.  Views are processed in passes of
 // BP_K views.  For every view of a pass one warp projects the 8 tile corners,
 // takes the bounding box of the taps the tile can touch (+1 pixel margin), and
 // one thread issues a 3D TMA load of a BW x BH detector box around it into
@@ -39,7 +39,7 @@
 //
 // Views whose u and w rows have a zero z coefficient -- every view of a
 // circular trajectory about the z axis -- take a column loop: 1/w, w^-2, u,
-// the u tap and its weight are then the same for the thread's 16 voxels and
+// the u tap and its weight are then the same for the thread's voxels and
 // are computed once, and v steps along the column as one FMA from its value
 // at the column base (within a few ulp of the general loop's per-voxel
 // v = (P1 . x) / w).
@@ -57,27 +57,30 @@ namespace {
 
 constexpr int TB_X = 32;
 constexpr int TB_Y = 8;
-constexpr int TB_Z = 16;  // voxels per thread along z
-constexpr int BP_K = 4;  // views per pass
-constexpr int BOX_W = 72;  // 72-element rows shift banks between rows (64 would alias them)
-constexpr int BOX_H = 24;
-constexpr int BOX_ELEMS = BOX_W * BOX_H;
-// Paired boxes (16-bit sinograms given a workspace for the paired copy):
-// 32-bit elements (tap u, tap u + 1), 68-word rows (4 banks of shift per row)
-constexpr int BOX_WP = 68;
 
-// The staged box of a sinogram type: element type, row length, TMA x
-// alignment (elements) and the paired copy's column offset (element u + 1
-// holds taps u and u + 1; element 0 holds a zero tap -1 and tap 0).
-template <typename T, bool PAIRED>
+// The staged box of a sinogram type: element type, row length (shifting banks
+// between rows: 64 would alias them), rows, TMA x alignment (elements) and
+// column offset, with the voxels per thread along z and the views per pass.
+// Paired boxes (16-bit sinograms given a workspace for the paired copy) hold
+// 32-bit elements: element u + 1 holds taps u and u + 1, element 0 a zero tap -1
+// and tap 0.
+// TALL: columns of 32 voxels over 48 rows, which halve a thread's work per view
+// (512^3, FP16: 31.1 -> 29.1 ms).  Taken for 16-bit sinograms of volumes with many
+// voxels per detector pixel (many_voxels_per_pixel), whether the paired copy
+// exists or not, so a result does not depend on the workspace.  The others keep
+// 16 over 24: with fewer, larger tiles small volumes run out of blocks, and FP32
+// boxes leave room for 3 blocks per SM (512^3: 30.97 against 30.96 ms).
+template <typename T, bool PAIRED, bool TALL>
 struct BoxLayout {
     using E = T;
-    static constexpr int W = BOX_W, ALIGN = 16 / (int)sizeof(T), OFF = 0;
+    static constexpr int W = 72, ALIGN = 16 / (int)sizeof(T), OFF = 0;
+    static constexpr int H = TALL ? 48 : 24, TB_Z = TALL ? 32 : 16, BP_K = TALL ? 2 : 4;
 };
 template <typename T>
-struct BoxLayout<T, true> {
+struct BoxLayout<T, true, true> {
     using E = unsigned;
-    static constexpr int W = BOX_WP, ALIGN = 4, OFF = 1;
+    static constexpr int W = 68, ALIGN = 4, OFF = 1;
+    static constexpr int H = 48, TB_Z = 32, BP_K = 2;
 };
 
 enum ViewMode : int { MODE_SMEM = 0, MODE_GLOBAL = 1, MODE_SKIP = 2 };
@@ -130,8 +133,8 @@ __device__ __forceinline__ float pair_ulerp<__nv_bfloat16>(unsigned w, float t)
     const float a = __uint_as_float(w << 16);
     return fmaf(t, sub_f32_bf16<true>(w, a), a);
 }
-template <typename T, bool PAIRED>
-__device__ __forceinline__ float box_ulerp(const typename BoxLayout<T, PAIRED>::E *p, float t)
+template <typename T, bool PAIRED, typename E>
+__device__ __forceinline__ float box_ulerp(const E *p, float t)
 {
     if constexpr (PAIRED)
         return pair_ulerp<T>(*p, t);  // 16-bit sinograms only
@@ -170,14 +173,15 @@ __device__ __forceinline__ float interp_global(const T *__restrict__ sino, float
 #endif
 
 // Computes the metadata of one pass (warp 0 only): lane = k * 8 + corner.
-template <typename T, bool PAIRED>
+template <typename T, bool PAIRED, bool TALL>
 __device__ __forceinline__ void pass_meta(ViewMeta *meta, const ConeBpView *__restrict__ pv, int n_first, int n_proj,
                                           int i0, int j0, int k0, int W, int H)
 {
+    using L = BoxLayout<T, PAIRED, TALL>;
     const int lane = threadIdx.x & 31;
     const int k = lane >> 3, c = lane & 7;
     const int n = n_first + k;
-    const bool live = n < n_proj;
+    const bool live = k < L::BP_K && n < n_proj;
     float4 r0 = make_float4(0, 0, 0, 0), r1 = r0, r2 = make_float4(0, 0, 0, 1);
     if (live) {
         r0 = __ldg(&pv[n].row[0]);
@@ -186,7 +190,7 @@ __device__ __forceinline__ void pass_meta(ViewMeta *meta, const ConeBpView *__re
     }
     const float ci = (float)(i0 + ((c & 1) ? TB_X - 1 : 0));
     const float cj = (float)(j0 + ((c & 2) ? TB_Y - 1 : 0));
-    const float ck = (float)(k0 + ((c & 4) ? TB_Z - 1 : 0));
+    const float ck = (float)(k0 + ((c & 4) ? L::TB_Z - 1 : 0));
     const float un = fmaf(r0.x, ci, fmaf(r0.y, cj, fmaf(r0.z, ck, r0.w)));
     const float vn = fmaf(r1.x, ci, fmaf(r1.y, cj, fmaf(r1.z, ck, r1.w)));
     const float wn = fmaf(r2.x, ci, fmaf(r2.y, cj, fmaf(r2.z, ck, r2.w)));
@@ -220,13 +224,12 @@ __device__ __forceinline__ void pass_meta(ViewMeta *meta, const ConeBpView *__re
             } else {
                 // the box's first element, x = iu0 + OFF in the staged
                 // layout, on the TMA alignment
-                using L = BoxLayout<T, PAIRED>;
                 const int a = L::ALIGN, xo = x_lo + L::OFF;
                 iu0 = ((xo >= 0) ? (xo / a) * a : -(((-xo) + a - 1) / a) * a) - L::OFF;
                 iv0 = y_lo;
                 // elements up to x_hi (the unpaired box's taps) or x_hi - 1
                 // (the paired element x_hi - 1 holds tap x_hi)
-                const bool fits = (x_hi - L::OFF - iu0 + 1 <= L::W) && (y_hi - iv0 + 1 <= BOX_H);
+                const bool fits = (x_hi - L::OFF - iu0 + 1 <= L::W) && (y_hi - iv0 + 1 <= L::H);
                 const bool clear_of_quirk = (x_hi <= W - 1) && (y_hi <= H - 1);
                 if (fits && clear_of_quirk) mode = MODE_SMEM;
             }
@@ -241,7 +244,7 @@ __device__ __forceinline__ void pass_meta(ViewMeta *meta, const ConeBpView *__re
     }
 }
 
-template <typename T, typename Tout, bool PAIRED>
+template <typename T, typename Tout, bool PAIRED, bool TALL>
 __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED))
     cone_bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, const T *__restrict__ sino, Tout *__restrict__ vol,
                        const ConeBpView *__restrict__ views, const float *__restrict__ mult, int X, int Y, int Z,
@@ -252,8 +255,9 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED))
     // TMA destinations must be 128-byte aligned: round the base up (the
     // launch reserves 128 spare bytes); every tile is a multiple of 128 bytes
     unsigned char *tile_base = dyn_smem + ((128u - (smem_addr(dyn_smem) & 127u)) & 127u);
-    using E = typename BoxLayout<T, PAIRED>::E;
-    constexpr int BW = BoxLayout<T, PAIRED>::W, BE = BW * BOX_H;
+    using L = BoxLayout<T, PAIRED, TALL>;
+    using E = typename L::E;
+    constexpr int TB_Z = L::TB_Z, BP_K = L::BP_K, BW = L::W, BE = BW * L::H;
     E(*tiles)[BP_K][BE] = reinterpret_cast<E(*)[BP_K][BE]>(tile_base);  // [2][BP_K][BE]
     __shared__ __align__(16) ViewMeta meta[2][BP_K];
     __shared__ __align__(8) uint64_t full[2];
@@ -297,12 +301,12 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED))
         for (int k = 0; k < BP_K; ++k) {
             const int n = p * BP_K + k;
             if (n < n_proj && meta[s][k].mode == MODE_SMEM)
-                tma_load_3d(&tiles[s][k][0], &tmap, meta[s][k].iu0 + BoxLayout<T, PAIRED>::OFF, meta[s][k].iv0,
+                tma_load_3d(&tiles[s][k][0], &tmap, meta[s][k].iu0 + L::OFF, meta[s][k].iv0,
                             b * n_proj + n, &full[s]);
         }
     };
     if (warp == 0) {
-        pass_meta<T, PAIRED>(meta[0], pv, 0, n_proj, i0, j0, k0, W, H);
+        pass_meta<T, PAIRED, TALL>(meta[0], pv, 0, n_proj, i0, j0, k0, W, H);
         __syncwarp();
     }
     __syncthreads();
@@ -321,7 +325,7 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED))
         const int cur = p & 1, nxt = cur ^ 1;
         __syncthreads();  // pass p-1 is done with stage nxt
         if (warp == 0 && p + 1 < n_pass) {
-            pass_meta<T, PAIRED>(meta[nxt], pv, (p + 1) * BP_K, n_proj, i0, j0, k0, W, H);
+            pass_meta<T, PAIRED, TALL>(meta[nxt], pv, (p + 1) * BP_K, n_proj, i0, j0, k0, W, H);
             __syncwarp();
             if (tid == 0) issue(p + 1, nxt);
         }
@@ -529,49 +533,48 @@ inline int paired_row(int W)
     return (W + 1 + 3) / 4 * 4;
 }
 
-// whether a 16-bit sinogram's paired copy pays: the pairing pass costs about a
-// read and two writes of the sinogram and saves a shared-memory load per tap
-// pair, worth it when a detector pixel serves many voxel updates (512^3 on
-// 1024 x 768: 171, 31.8 against 32.5 ms; 256^3 on 512^2: 64, 4.26 against 4.08 ms)
-inline bool pairing_pays(int in_dtype, const Dims3D &d)
+// whether a 16-bit sinogram takes tall columns and, given room, a paired copy:
+// the pairing pass costs about a read and two writes of the sinogram and saves a
+// shared-memory load per tap pair, worth it when a detector pixel serves many
+// voxel updates (512^3 on 1024 x 768: 171, 31.8 against 32.5 ms; 256^3 on 512^2: 64,
+// 4.26 against 4.08 ms)
+inline bool many_voxels_per_pixel(int in_dtype, const Dims3D &d)
 {
     return dtype_size(in_dtype) == 2 && (long long)d.vol_x * d.vol_y * d.vol_z >= 100LL * d.det_h * d.det_w;
 }
 
 // `pitch`: elements between the staged rows
-template <typename Tin, typename Tout, bool PAIRED>
+template <typename Tin, typename Tout, bool PAIRED, bool TALL>
 cudaError_t launch_kernel(const void *sinogram, const void *staged, int pitch, void *volume, const Dims3D &d,
                           const ConeBpView *views, const float *mult, unsigned *err, int starve_last_pass,
                           cudaStream_t stream)
 {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
-    using L = BoxLayout<Tin, PAIRED>;
+    using L = BoxLayout<Tin, PAIRED, TALL>;
     using E = typename L::E;
     const cuuint64_t row = PAIRED ? (cuuint64_t)pitch : (cuuint64_t)d.det_w;
     CUtensorMap map;
     const cuuint64_t dims[3] = {row, (cuuint64_t)d.det_h, (cuuint64_t)d.n_proj * d.batch};
     const cuuint64_t strides[2] = {pitch * sizeof(E), (cuuint64_t)pitch * d.det_h * sizeof(E)};
-    const cuuint32_t box[3] = {(cuuint32_t)L::W, BOX_H, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)L::W, (cuuint32_t)L::H, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType type = PAIRED ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : tma_type<Tin>();
     CUresult r = enc(&map, type, 3, const_cast<void *>(staged), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    const int zblocks = (d.vol_z + TB_Z - 1) / TB_Z;
+    const int zblocks = (d.vol_z + L::TB_Z - 1) / L::TB_Z;
     const dim3 block(TB_X, TB_Y, 1);
     const dim3 grid((d.vol_x + TB_X - 1) / TB_X, (d.vol_y + TB_Y - 1) / TB_Y, zblocks * d.batch);
-    static_assert((BOX_ELEMS * sizeof(float)) % 128 == 0 && (BOX_ELEMS * 2) % 128 == 0 &&
-                      (BOX_WP * BOX_H * 4) % 128 == 0,
-                  "tile alignment");
-    const size_t smem = 2 * BP_K * (size_t)L::W * BOX_H * sizeof(E) + 128;
+    static_assert((L::W * L::H * sizeof(E)) % 128 == 0, "tile alignment");
+    const size_t smem = 2 * L::BP_K * (size_t)L::W * L::H * sizeof(E) + 128;
     // set on every launch: the attribute belongs to the current device's copy
     // of the kernel, and the call is a cheap host-side update
-    cudaError_t e = cudaFuncSetAttribute(cone_bp_tma_kernel<Tin, Tout, PAIRED>,
+    cudaError_t e = cudaFuncSetAttribute(cone_bp_tma_kernel<Tin, Tout, PAIRED, TALL>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    cone_bp_tma_kernel<Tin, Tout, PAIRED><<<grid, block, smem, stream>>>(
+    cone_bp_tma_kernel<Tin, Tout, PAIRED, TALL><<<grid, block, smem, stream>>>(
         map, (const Tin *)sinogram, (Tout *)volume, views, mult, d.vol_x, d.vol_y, d.vol_z, d.det_w, d.det_h, d.n_proj,
         d.geom_batch, err, starve_last_pass);
     return cudaGetLastError();
@@ -584,16 +587,24 @@ cudaError_t launch_typed(const void *sinogram, void *volume, int in_dtype, const
     const long long rows = (long long)d.batch * d.n_proj * d.det_h;
     const unsigned ygrid = (unsigned)(rows < 65535 ? rows : 65535);
     if constexpr (sizeof(Tin) == 2) {
-        if (copy && pairing_pays(in_dtype, d)) {
+        if (copy && many_voxels_per_pixel(in_dtype, d)) {
             const int Wp = paired_row(d.det_w);
             pair_sinogram_kernel<Tin><<<dim3((unsigned)((Wp + 255) / 256), ygrid), 256, 0, stream>>>(
                 (const Tin *)sinogram, (unsigned *)copy, d.det_w, Wp, rows);
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
-            return launch_kernel<Tin, Tout, true>(sinogram, copy, Wp, volume, d, views, mult, err, starve_last_pass,
-                                                  stream);
+            return launch_kernel<Tin, Tout, true, true>(sinogram, copy, Wp, volume, d, views, mult, err,
+                                                        starve_last_pass, stream);
         }
     }
+    auto launch_unpaired = [&](const void *staged, int pitch) {
+        if constexpr (sizeof(Tin) == 2)
+            if (many_voxels_per_pixel(in_dtype, d))
+                return launch_kernel<Tin, Tout, false, true>(sinogram, staged, pitch, volume, d, views, mult, err,
+                                                             starve_last_pass, stream);
+        return launch_kernel<Tin, Tout, false, false>(sinogram, staged, pitch, volume, d, views, mult, err,
+                                                      starve_last_pass, stream);
+    };
     if (copy) {
         const int Wp = pitched_row(d.det_w, sizeof(Tin));
         const int chunks = Wp / (16 / (int)sizeof(Tin));
@@ -601,11 +612,9 @@ cudaError_t launch_typed(const void *sinogram, void *volume, int in_dtype, const
             (const Tin *)sinogram, (Tin *)copy, d.det_w, Wp, rows);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        return launch_kernel<Tin, Tout, false>(sinogram, copy, Wp, volume, d, views, mult, err, starve_last_pass,
-                                               stream);
+        return launch_unpaired(copy, Wp);
     }
-    return launch_kernel<Tin, Tout, false>(sinogram, sinogram, d.det_w, volume, d, views, mult, err, starve_last_pass,
-                                           stream);
+    return launch_unpaired(sinogram, d.det_w);
 }
 
 }  // namespace
@@ -618,6 +627,7 @@ bool cone_bp_tma_supported(const void *sinogram, int in_dtype, const Dims3D &d, 
     const size_t e = dtype_size(in_dtype);
     if (e == 0) return false;
     if (!copy && (((uintptr_t)sinogram % 16) != 0 || ((size_t)d.det_w * e) % 16 != 0)) return false;
+    constexpr int TB_Z = BoxLayout<float, false, false>::TB_Z;  // the shorter columns
     const long long zb = (d.vol_z + TB_Z - 1) / TB_Z;
     if (zb * d.batch > 65535 || (d.vol_y + TB_Y - 1) / TB_Y > 65535) return false;
     if ((long long)d.n_proj * d.batch >= (1LL << 31)) return false;
@@ -637,7 +647,7 @@ size_t cone_bp_tma_copy_bytes(int in_dtype, const Dims3D &d)
 {
     const size_t e = dtype_size(in_dtype), rows = (size_t)d.batch * d.n_proj * d.det_h;
     if (e == 0) return 0;
-    if (pairing_pays(in_dtype, d)) return rows * (size_t)paired_row(d.det_w) * sizeof(unsigned);
+    if (many_voxels_per_pixel(in_dtype, d)) return rows * (size_t)paired_row(d.det_w) * sizeof(unsigned);
     return ((size_t)d.det_w * e) % 16 != 0 ? rows * (size_t)pitched_row(d.det_w, e) * e : 0;
 }
 

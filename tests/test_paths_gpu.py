@@ -316,3 +316,28 @@ def test_texture_fill_widths(cuda, width, dtype):
             for b in range(2):
                 one = op(x[b:b + 1].clone(), out_shape, *geo.args(), hardware_interp=True)
                 assert torch.equal(one[0], both[b])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vol_shape", [(33, 40, 64), (31, 41, 65), (70, 24, 40)])
+def test_cone_backprojection_tall_columns(cuda, vol_shape, dtype):
+    """16-bit sinograms of many voxels per detector pixel take columns of 32
+    voxels, with the paired copy and without it: the same bits, for depths on
+    either side of a tile, and the oracle's values."""
+    geo = geometry.ConeBeam3D(vol_shape, (1.0, 1.0, 1.0), (20, 32), (4.0, 4.0), 9, 160.0, 260.0)
+    assert np.prod(vol_shape) >= 100 * 20 * 32
+    sino = t(noise(61, (1,) + geo.detector_shape), cuda, dtype)
+    gc = pl.ops.GeometryCone(1, cuda, *geo.args(), geo.detector_shape[0])
+    code = pl.ops.storage_code(dtype)
+    outs = []
+    for batch in (1, 0):  # with the paired copy, and the views' part alone
+        n = _capi.workspace_size("pyronn_cone_backprojection3d", batch, *geo.detector_shape, *vol_shape, code, 0, 1)
+        ws = torch.empty(n, dtype=torch.uint8, device=cuda)
+        out = torch.full((1,) + vol_shape, 7.0, device=cuda)
+        _capi.call("pyronn_cone_backprojection3d", sino.data_ptr(), out.data_ptr(), code, 0, 0, 1,
+                   *geo.detector_shape, *vol_shape, *gc.pointers(), 1, ws.data_ptr(), n,
+                   torch.cuda.current_stream().cuda_stream)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    ref = oracle.cone_backprojection3d(sino.float().cpu().numpy(), vol_shape, *geo.args())
+    assert rel_l2(outs[0].cpu().numpy(), ref) < 1e-5
