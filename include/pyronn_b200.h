@@ -333,8 +333,11 @@ PYRONN_API int pyronn_circular_ray_vectors_2d(float *ray_vectors, int n_proj, do
  * the same buffer (of one storage type).  det_w <= PYRONN_FDK_MAX_WIDTH.  Rows
  * of up to 2048 pixels go through FP32 Fourier transforms of the row
  * differences (about 1.5e-7 relative of the exact filter), wider ones are
- * direct FP32 sums.  A row holding infinities or NaNs comes back as NaNs;
- * others are not affected by it.
+ * direct FP32 sums, as are rows with a pixel far above any line integral (two
+ * neighbours 2^64 apart, 2^14 for FP16 input: a masked pixel, an infinity).  An
+ * infinity or a NaN reaches the outputs its non-zero taps join it to; with
+ * distinct, 16-byte aligned buffers and det_w a multiple of 4 up to 2048 the
+ * whole row comes back as NaNs.  Other rows are not affected by it.
  * ------------------------------------------------------------------------- */
 #define PYRONN_FILTER_RAM_LAK 0
 #define PYRONN_FILTER_SHEPP_LOGAN 1

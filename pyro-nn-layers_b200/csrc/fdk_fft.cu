@@ -16,8 +16,13 @@
 // Ram-Lak k[m] = (1 / (pi^2 tau)) sum of 1/i^2 over odd i > m, a trigamma value
 // (Abramowitz & Stegun 6.4.6, 6.4.12); Shepp-Logan 1 / (pi^2 tau (2 m + 1)).
 // Rows of a pair are scaled by powers of two to a common magnitude, so neither
-// takes rounding errors of the other's size, and a row holding infinities or
-// NaNs is transformed as zeros and written as NaNs.
+// takes rounding errors of the other's size.
+// A row with a difference outside the transforms' range (peak_limit: an
+// infinity, a NaN, a difference that overflows, a masked pixel of the storage
+// type's lowest value) is transformed as zeros and summed directly instead
+// (direct_rows): a transform spreads its rounding, 1.5e-7 of the row's largest
+// difference, over all outputs, while half of the Ram-Lak taps are zero and
+// leave the outputs they do not join to such a pixel as they are.
 //
 // The transform: N = 16 * 16 * R3, decimation in frequency forward (radices 16,
 // 16, R3, results in digit-reversed order), the product, and decimation in time
@@ -28,7 +33,10 @@
 // Toeplitz product on the tensor cores (O(W^2) operations): 276 k rows of 1024
 // pixels, FP16 in, FP32 out, 4.72 -> 1.67 ms; 184 k of 512, 0.93 -> 0.58; 26 k FP32
 // rows of 2000, 1.65 -> 0.37.
+#include <type_traits>
+
 #include "common.cuh"
+#include "fdk_taps.cuh"
 #include "internal.h"
 
 namespace pyronn {
@@ -194,12 +202,78 @@ __device__ __forceinline__ void inverse(float2 (&x)[16], float2 *buf, const floa
     dft<true, 16>(x);
 }
 
+// The bits of the least magnitude of a row's differences that takes the row out
+// of the transforms' range: 2^64, 2^14 for FP16 storage (whose lowest value is
+// -65504), both far above any line integral.
+template <typename Tin>
+__host__ __device__ constexpr unsigned peak_limit()
+{
+    return (127u + (std::is_same<Tin, __half>::value ? 14u : 64u)) << 23;
+}
+
+// The Feldkamp cosine weight of column j on a row at height vv.
+__device__ __forceinline__ float cosine_weight(int j, float vv, float sdd, float du, float cu)
+{
+    const float uu = ((float)j - cu) * du;
+    return sdd * rsqrtf(fmaf(sdd, sdd, fmaf(uu, uu, vv * vv)));
+}
+
+// The rows `first` (if bad_a) and `first` + 1 (if bad_b) of a pair by direct
+// FP32 sums over the taps that are not zero, in the order of fdk.cu's kernel.
+// nan_rows: a row that holds an infinity or a NaN is written as NaNs.  Called by
+// the whole block (`scratch`: a word per warp); every group has the row and the
+// taps in its own `buf`.
+template <typename Tin, typename Tout, int R3>
+__device__ __noinline__ void direct_rows(const Tin *in, Tout *out, long long first, bool bad_a, bool bad_b, int det_h,
+                                         int W, float sdd, float dv, float du, float cv, float cu, int kind,
+                                         int weight_output, int nan_rows, float2 *buf, unsigned *scratch)
+{
+    using P = Plan<R3>;
+    constexpr int M = P::M, WARPS = M / 32;
+    const int tid = threadIdx.x, grp = tid / M, t = tid % M;
+    float *g = reinterpret_cast<float *>(buf), *taps = g + P::N;  // W <= N / 2 of each; buf is 2 N floats and more
+    for (int r = 0; r < 2; ++r) {
+        const bool bad = r == 0 ? bad_a : bad_b;
+        const float vv = ((float)(int)((first + r) % det_h) - cv) * dv;
+        const Tin *row = in + (first + r) * W;
+        bool nonfinite = false;
+        if (bad)
+            for (int j = t; j < W; j += M) {
+                float x = load_as_float(row + j);
+                if (!weight_output && sdd > 0.0f) x *= cosine_weight(j, vv, sdd, du, cu);
+                nonfinite |= !isfinite(x);
+                g[j] = x;
+                taps[j] = fdk_tap(kind, j, du);
+            }
+        const bool warp_nonfinite = __any_sync(0xffffffffu, nonfinite);
+        if ((tid & 31) == 0) scratch[tid / 32] = warp_nonfinite;
+        __syncthreads();  // the row is read completely before it is written
+        if (bad) {
+            bool all_nan = false;
+            for (int w = 0; w < WARPS; ++w) all_nan |= nan_rows && scratch[grp * WARPS + w];
+            for (int j = t; j < W; j += M) {
+                float q = 0.0f;
+                if (kind == PYRONN_FILTER_RAM_LAK) {  // odd offsets and the centre
+                    for (int k = (j + 1) & 1; k < W; k += 2) q = fmaf(taps[abs(j - k)], g[k], q);
+                    q = fmaf(taps[0], g[j], q);
+                } else {
+                    for (int k = 0; k < W; ++k) q = fmaf(taps[abs(j - k)], g[k], q);
+                }
+                if (all_nan) q = __uint_as_float(0x7fffffffu);
+                if (weight_output && sdd > 0.0f) q *= cosine_weight(j, vv, sdd, du, cu);
+                store_from_float(out + (first + r) * W + j, q);
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // in and out may be the same buffer: a pair's rows are read completely before
 // they are written, by the threads that own them.
 template <typename Tin, typename Tout, int R3>
 __global__ void __launch_bounds__(FFT_THREADS, FFT_BLOCKS)
     fdk_filter_fft_kernel(const Tin *in, Tout *out, long long rows, int det_h, int W, float sdd, float dv, float du,
-                          float cv, float cu, int kind, int weight_output)
+                          float cv, float cu, int kind, int weight_output, int nan_rows)
 {
     using P = Plan<R3>;
     constexpr int M = P::M, WARPS = M / 32;
@@ -244,10 +318,7 @@ __global__ void __launch_bounds__(FFT_THREADS, FFT_BLOCKS)
         const bool live_a = ra < rows, live_b = ra + 1 < rows;
         const float va = ((float)(int)(ra % det_h) - cv) * dv, vb = ((float)(int)((ra + 1) % det_h) - cv) * dv;
         const Tin *ia = in + ra * W, *ib = ia + W;
-        auto weight = [&](int j, float vv) {
-            const float uu = ((float)j - cu) * du;
-            return sdd * rsqrtf(fmaf(sdd, sdd, fmaf(uu, uu, vv * vv)));
-        };
+        auto weight = [&](int j, float vv) { return cosine_weight(j, vv, sdd, du, cu); };
         // the rows' values, then their differences
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -284,10 +355,14 @@ __global__ void __launch_bounds__(FFT_THREADS, FFT_BLOCKS)
             pb = max(pb, peak[1][grp * WARPS + w]);
         }
         // powers of two that bring the largest difference into [1, 2)
-        const unsigned ea = pa >> 23, eb = pb >> 23;  // 0: zero (or flushed), 255: not finite
-        const bool bad_a = ea == 255u, bad_b = eb == 255u;
-        const float sa = ea == 0u || bad_a ? 1.0f : __uint_as_float(max(254u - ea, 1u) << 23);
-        const float sb = eb == 0u || bad_b ? 1.0f : __uint_as_float(max(254u - eb, 1u) << 23);
+        const unsigned ea = pa >> 23, eb = pb >> 23;  // 0: zero (or flushed)
+        const bool bad_a = pa >= peak_limit<Tin>(), bad_b = pb >= peak_limit<Tin>();
+        const float sa = ea == 0u || bad_a ? 1.0f : __uint_as_float((254u - ea) << 23);
+        const float sb = eb == 0u || bad_b ? 1.0f : __uint_as_float((254u - eb) << 23);
+        // the factors back: zero for a row of zeros, which stays zeros; NaN marks
+        // a row that is summed directly
+        const float nan = __uint_as_float(0x7fffffffu);
+        const float ua = bad_a ? nan : (ea == 0u ? 0.0f : 1.0f / sa), ub = bad_b ? nan : (eb == 0u ? 0.0f : 1.0f / sb);
 #pragma unroll
         for (int k = 0; k < 9; ++k) x[k] = make_float2(bad_a ? 0.0f : x[k].x * sa, bad_b ? 0.0f : x[k].y * sb);
 #pragma unroll
@@ -299,9 +374,6 @@ __global__ void __launch_bounds__(FFT_THREADS, FFT_BLOCKS)
             x[k] = cmul<false>(x[k], w.x, w.y);
         }
         inverse<R3>(x, buf, tw1, tw2, t);
-        const float nan = __uint_as_float(0x7fffffffu);
-        // (a row of zeros stays zeros)
-        const float ua = bad_a ? nan : (ea == 0u ? 0.0f : 1.0f / sa), ub = bad_b ? nan : (eb == 0u ? 0.0f : 1.0f / sb);
         Tout *oa = out + ra * W, *ob = oa + W;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -309,17 +381,20 @@ __global__ void __launch_bounds__(FFT_THREADS, FFT_BLOCKS)
             if (j < W) {
                 float qa = x[k].x * ua, qb = x[k].y * ub;
                 if (weight_output && sdd > 0.0f) qa *= weight(j, va), qb *= weight(j, vb);
-                if (live_a) store_from_float(oa + j, qa);
-                if (live_b) store_from_float(ob + j, qb);
+                if (live_a && !isnan(ua)) store_from_float(oa + j, qa);
+                if (live_b && !isnan(ub)) store_from_float(ob + j, qb);
             }
         }
-        __syncthreads();  // every thread is done with the exchange buffer
+        // every thread is done with the exchange buffer
+        if (__syncthreads_or(isnan(ua) || isnan(ub)))
+            direct_rows<Tin, Tout, R3>(in, out, 2 * (p0 + grp), isnan(ua), isnan(ub), det_h, W, sdd, dv, du, cv, cu, kind,
+                                       weight_output, nan_rows, buf, peak[0]);
     }
 }
 
 template <typename Tin, typename Tout, int R3>
 cudaError_t launch_plan(const void *in, void *out, long long rows, int det_h, int W, float sdd, float dv, float du,
-                        float cv, float cu, int kind, int weight_output, cudaStream_t stream)
+                        float cv, float cu, int kind, int weight_output, int nan_rows, cudaStream_t stream)
 {
     using P = Plan<R3>;
     auto kernel = fdk_filter_fft_kernel<Tin, Tout, R3>;
@@ -329,7 +404,7 @@ cudaError_t launch_plan(const void *in, void *out, long long rows, int det_h, in
     const long long groups = ((rows + 1) / 2 + P::PAIRS - 1) / P::PAIRS;
     const unsigned grid = (unsigned)(groups < 148 * FFT_BLOCKS ? groups : 148 * FFT_BLOCKS);
     kernel<<<grid, FFT_THREADS, P::SMEM, stream>>>((const Tin *)in, (Tout *)out, rows, det_h, W, sdd, dv, du, cv, cu,
-                                                   kind, weight_output);
+                                                   kind, weight_output, nan_rows);
     return cudaGetLastError();
 }
 
@@ -344,6 +419,12 @@ cudaError_t launch_fdk_filter_fft(const void *in, void *out, int in_dtype, int o
                                   int W, float sdd, float dv, float du, float cv, float cu, int kind,
                                   int weight_output, cudaStream_t stream)
 {
+    // rows with infinities or NaNs: NaNs throughout on distinct, aligned buffers
+    // of quad rows, the direct sums' in every other call
+    const char *ib = (const char *)in, *ob = (const char *)out;
+    const size_t n = (size_t)rows * (size_t)W;
+    const bool overlap = ib < ob + n * dtype_size(out_dtype) && ob < ib + n * dtype_size(in_dtype);
+    const int nan_rows = W % 4 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 && !overlap;
     return dispatch_dtypes(in_dtype, out_dtype, [&](auto tin, auto tout) -> cudaError_t {
         using Tin = typename decltype(tin)::type;
         using Tout = typename decltype(tout)::type;
@@ -351,7 +432,7 @@ cudaError_t launch_fdk_filter_fft(const void *in, void *out, int in_dtype, int o
                       : W <= 512  ? launch_plan<Tin, Tout, 4>
                       : W <= 1024 ? launch_plan<Tin, Tout, 8>
                                   : launch_plan<Tin, Tout, 16>;
-        return launch(in, out, rows, det_h, W, sdd, dv, du, cv, cu, kind, weight_output, stream);
+        return launch(in, out, rows, det_h, W, sdd, dv, du, cv, cu, kind, weight_output, nan_rows, stream);
     });
 }
 
