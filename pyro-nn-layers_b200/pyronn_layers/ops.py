@@ -74,39 +74,80 @@ _HOST_GEOM_CACHE: "collections.OrderedDict" = collections.OrderedDict()
 _HOST_GEOM_CACHE_SIZE = 64
 
 
+class _HostArray:
+    """A host array as float32, with its content as a key and, once it is on a
+    device, the streams its copy there is recorded on."""
+
+    __slots__ = ("array", "key", "streams")
+
+    def __init__(self, t):
+        a = t.detach().numpy() if isinstance(t, torch.Tensor) else t
+        self.array = a = np.ascontiguousarray(a, dtype=np.float32)
+        self.key = (a.shape, a.tobytes() if a.nbytes <= 4096 else hashlib.blake2b(a.data, digest_size=16).digest())
+
+
 def _host_geometry_on_device(t, device) -> torch.Tensor:
-    a = np.ascontiguousarray(t.numpy() if isinstance(t, torch.Tensor) else np.asarray(t), dtype=np.float32)
+    h = t if isinstance(t, _HostArray) else _HostArray(t)
     dev = torch.device(device)
     if dev.type == "cuda" and dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
-    key = (str(dev), a.shape, hashlib.blake2b(a.tobytes(), digest_size=16).digest())
+    key = (dev, h.key)
     hit = _HOST_GEOM_CACHE.get(key)
     if hit is not None:
-        _HOST_GEOM_CACHE.move_to_end(key)
-        return hit
-    d = torch.from_numpy(a.copy()).to(dev)
+        d, h.streams = hit
+        _touch(_HOST_GEOM_CACHE, key)
+        if h is not t:  # (a pack's tensors are recorded by its launches)
+            _used_on_current_stream((d,), h.streams, dev)
+        return d
+    d = torch.from_numpy(h.array.copy()).to(dev)
+    h.streams = set()
     if dev.type == "cuda":
         # the copy is complete before any stream uses the cached tensor
         torch.cuda.current_stream(dev).synchronize()
-    _HOST_GEOM_CACHE[key] = d
-    _evict(_HOST_GEOM_CACHE, dev)
+        h.streams.add(_stream(dev))
+    _HOST_GEOM_CACHE[key] = (d, h.streams)
+    _evict(_HOST_GEOM_CACHE)
     return d
 
 
-def _evict(cache, dev) -> None:
-    """Bounds a geometry cache; a dropped entry's memory may be read by work
-    queued on any stream, which is waited for first."""
-    if len(cache) > _HOST_GEOM_CACHE_SIZE:
-        if dev.type == "cuda":
-            torch.cuda.synchronize(dev)
-        while len(cache) > _HOST_GEOM_CACHE_SIZE:
+def _touch(cache, key) -> None:
+    try:
+        cache.move_to_end(key)
+    except KeyError:  # evicted by another thread since
+        pass
+
+
+def _evict(cache) -> None:
+    """Bounds a geometry cache.  Waits for nothing: the memory of a dropped
+    entry is reused only after the work queued on it (_used_on_current_stream),
+    whoever held it last."""
+    while len(cache) > _HOST_GEOM_CACHE_SIZE:
+        try:
             cache.popitem(last=False)
+        except KeyError:  # emptied by another thread
+            return
+
+
+def _used_on_current_stream(tensors, streams, device) -> None:
+    """Tells the allocator, once per stream, that cached geometry is read by work
+    on the current stream of its device; `streams` holds the streams it knows
+    of.  (A captured graph's reads are not on the capturing stream: nothing is
+    recorded under a capture.)"""
+    if device.type != "cuda":
+        return
+    raw = _stream(device)
+    if raw in streams or torch.cuda.is_current_stream_capturing():
+        return
+    stream = torch.cuda.current_stream(device)
+    for t in tensors:
+        t.record_stream(stream)
+    streams.add(raw)
 
 
 def _geom(t, batch: int, row_shape: Sequence[int], device, what: str):
     """Returns (contiguous float32 tensor [g, *row_shape] on device, g)."""
     if not (isinstance(t, torch.Tensor) and t.device.type == "cuda"):
-        t = _host_geometry_on_device(t.detach() if isinstance(t, torch.Tensor) else t, device)
+        t = _host_geometry_on_device(t, device)
     t = torch.as_tensor(t, dtype=torch.float32)
     row_numel = 1
     for s in row_shape:
@@ -147,6 +188,14 @@ def _check_data(x: torch.Tensor, ndim: int, what: str):
 def _stream(device) -> int:
     index = device.index if device.index is not None else torch.cuda.current_device()
     return torch._C._cuda_getCurrentRawStream(index)
+
+
+def _launch_stream(geo, device) -> int:
+    """The current stream, for a launch that reads geo."""
+    raw = _stream(device)
+    if geo.streams is not None and raw not in geo.streams:
+        _used_on_current_stream(geo.tensors(), geo.streams, device)
+    return raw
 
 
 def _on_device(device):
@@ -248,6 +297,7 @@ class Geometry2D:
             gs += [g6, g7]
         g = _common_g(*gs)
         self.g = g
+        self.expanded = min(gs) != g
         self.volume_origin = _expand(vo, g)
         self.detector_origin = _expand(do, g)
         self.volume_spacing = _expand(vs, g)
@@ -256,6 +306,11 @@ class Geometry2D:
         if self.fan:
             self.sid = _expand(si, g)
             self.sdd = _expand(sd, g)
+        self.streams = None  # of a cached pack: the streams its tensors are recorded on
+
+    def tensors(self):
+        t = [self.volume_origin, self.detector_origin, self.volume_spacing, self.detector_spacing, self.rays]
+        return t + [self.sid, self.sdd] if self.fan else t
 
     def pointers(self):
         p = [self.volume_origin.data_ptr(), self.detector_origin.data_ptr(), self.volume_spacing.data_ptr(),
@@ -278,12 +333,18 @@ class GeometryCone:
         mu, g5 = _geom(projection_multiplier, batch, (1,), device, "projection_multiplier")
         g = _common_g(g1, g2, g3, g4, g5)
         self.g = g
+        self.expanded = min(g1, g2, g3, g4, g5) != g
         self.n_proj = n_proj
         self.volume_origin = _expand(vo, g)
         self.volume_spacing = _expand(vs, g)
         self.projection_matrices = _expand(pm, g)
         self.step_size = _expand(st, g)
         self.projection_multiplier = _expand(mu, g)
+        self.streams = None  # of a cached pack: the streams its tensors are recorded on
+
+    def tensors(self):
+        return [self.volume_origin, self.volume_spacing, self.projection_matrices, self.step_size,
+                self.projection_multiplier]
 
     def pointers(self):
         return [self.volume_origin.data_ptr(), self.volume_spacing.data_ptr(),
@@ -299,46 +360,41 @@ _PACKS: "collections.OrderedDict" = collections.OrderedDict()
 
 
 def _pack(cls, batch: int, device, n_proj: int, arrays, build):
-    key = [cls, batch, n_proj, device]
-    for a in arrays:
-        if a is None:
-            key.append(None)
-            continue
-        if isinstance(a, torch.Tensor):
-            if a.is_cuda:
-                return build()
-            a = a.detach().numpy()
-        a = np.ascontiguousarray(a, dtype=np.float32)
-        key.append(a.shape)
-        key.append(a.tobytes() if a.nbytes <= 4096 else hashlib.blake2b(a.data, digest_size=16).digest())
-    key = tuple(key)
+    if any(isinstance(a, torch.Tensor) and a.is_cuda for a in arrays):
+        return build(*arrays)
+    arrays = [None if a is None else _HostArray(a) for a in arrays]
+    key = (cls, batch, n_proj, device, *(a and a.key for a in arrays))
     hit = _PACKS.get(key)
     if hit is None:
         if device.type == "cuda" and torch.cuda.is_current_stream_capturing():
-            return build()  # what a capture computes exists only when its graph is replayed
-        hit = build()
+            return build(*arrays)  # what a capture computes exists only when its graph is replayed
+        hit = build(*arrays)
+        hit.streams = set()
         if device.type == "cuda":
-            # expanded rows are complete before any stream uses the pack
-            torch.cuda.current_stream(device).synchronize()
+            if hit.expanded:
+                # the expanded rows are complete before any stream uses the pack
+                torch.cuda.current_stream(device).synchronize()
+            raw = _stream(device)
+            if all(a is None or raw in a.streams for a in arrays):
+                hit.streams.add(raw)
         _PACKS[key] = hit
-        _evict(_PACKS, device)
+        _evict(_PACKS)
     else:
-        try:
-            _PACKS.move_to_end(key)
-        except KeyError:  # evicted by another thread since
-            pass
+        _touch(_PACKS, key)
     return hit
 
 
 def _geometry_2d(x, n_proj, volume_origin, detector_origin, volume_spacing, detector_spacing, rays, sid=None, sdd=None):
-    arrays = (volume_origin, detector_origin, volume_spacing, detector_spacing, rays, sid, sdd)
-    return _pack(Geometry2D, x.shape[0], x.device, n_proj, arrays,
-                 lambda: Geometry2D(x.shape[0], x.device, *arrays[:5], n_proj, sid, sdd))
+    def build(vo, do, vs, ds, rv, si, sd):
+        return Geometry2D(x.shape[0], x.device, vo, do, vs, ds, rv, n_proj, si, sd)
+    return _pack(Geometry2D, x.shape[0], x.device, n_proj,
+                 (volume_origin, detector_origin, volume_spacing, detector_spacing, rays, sid, sdd), build)
 
 
 def _geometry_cone(x, n_proj, *arrays):
-    return _pack(GeometryCone, x.shape[0], x.device, n_proj, arrays,
-                 lambda: GeometryCone(x.shape[0], x.device, *arrays, n_proj))
+    def build(*a):
+        return GeometryCone(x.shape[0], x.device, *a, n_proj)
+    return _pack(GeometryCone, x.shape[0], x.device, n_proj, arrays, build)
 
 
 # ------------------------------------------------------------- raw launches
@@ -375,7 +431,7 @@ def _run_2d(forward: bool, x: torch.Tensor, out_dims, geo: Geometry2D, out_dtype
         ws = []
     with _on_device(dev):
         _capi.call(fn, x.data_ptr(), out.data_ptr(), storage_code(x.dtype), storage_code(od), *dims,
-                   *geo.pointers(), geo.g, *ws, _stream(dev))
+                   *geo.pointers(), geo.g, *ws, _launch_stream(geo, dev))
     return out
 
 
@@ -418,7 +474,7 @@ def _run_cone(forward: bool, x: torch.Tensor, out_dims, geo: GeometryCone, hardw
     with _on_device(dev):
         _capi.call(fn, x.data_ptr(), out.data_ptr(), storage_code(x.dtype), storage_code(od),
                    int(bool(hardware_interp)), *dims, *geo.pointers(), geo.g, workspace.data_ptr(),
-                   workspace.numel(), _stream(dev))
+                   workspace.numel(), _launch_stream(geo, dev))
         if not forward and not hardware_interp:
             note_workspace_error(workspace, dev)  # the TMA-staged path's bounded waits
     return out
@@ -437,7 +493,7 @@ def _run_matched(p: torch.Tensor, vol_dims, geo: GeometryCone) -> torch.Tensor:
         _capi.call(fn, p.data_ptr(), out.data_ptr(), storage_code(p.dtype), batch, n_proj, det_h, det_w, vol_z, vol_y,
                    vol_x, geo.volume_origin.data_ptr(), geo.volume_spacing.data_ptr(),
                    geo.projection_matrices.data_ptr(), geo.step_size.data_ptr(), geo.g, ws.data_ptr(), ws.numel(),
-                   _stream(dev))
+                   _launch_stream(geo, dev))
     return out
 
 
