@@ -359,16 +359,21 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED))
                     // rows of voxels z and z + 1 differ by 0 or 1: the pair
                     // reads rows r, r + 1, r + 2 once (three u lerps for two
                     // voxels instead of four) and gives each voxel its two;
-                    // positions, floors, v lerps and sums of the pair run on
-                    // the packed FP32 instructions (one issue slot for both,
-                    // at half the rate: 512^3, FP16, 31.7 -> 31.1 ms; FP32
-                    // 256^3, 3.91 -> 3.78 ms)
+                    // floors, v lerps and sums of the pair run on the packed
+                    // FP32 instructions (one issue slot for both, at half the
+                    // rate: 512^3, FP16, 31.7 -> 31.1 ms).  Each position is one
+                    // FMA from the column base: sums of 2 dlv in their place
+                    // drift by up to 15 roundings of one sign in a column of 32
+                    // (512^3: FP16 29.05 ms with the sums, 28.89 with the FMAs;
+                    // FP32 30.9 / 31.4; 256^3, FP32, 3.77 / 3.86).
+                    // The v lerp a + t (b - a) rounds as often as lerp_ref, which
+                    // needs -t as well (30.5 ms).
                     constexpr float MAGIC = 12582912.0f;  // floor_frac's, 1.5 * 2^23
                     const float2 minus1 = make_float2(-1.0f, -1.0f);
-                    const float2 rw2p = make_float2(rw2, rw2), dl2 = make_float2(dlv + dlv, dlv + dlv);
-                    float2 l = make_float2(lv0, lv0 + dlv);
+                    const float2 rw2p = make_float2(rw2, rw2);
 #pragma unroll
                     for (int z = 0; z < TB_Z; z += 2) {
+                        const float2 l = make_float2(fmaf((float)z, dlv, lv0), fmaf((float)(z + 1), dlv, lv0));
                         const float2 fl = __fadd2_rd(l, make_float2(MAGIC, MAGIC));
                         const float2 fr = __ffma2_rn(__fadd2_rn(fl, make_float2(-MAGIC, -MAGIC)), minus1, l);
                         const int ra = __float_as_int(fl.x);
@@ -382,7 +387,6 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED))
                         const float2 v = __ffma2_rn(fr, __ffma2_rn(a, minus1, b), a);
                         const float2 s = __ffma2_rn(v, rw2p, make_float2(acc[z], acc[z + 1]));
                         acc[z] = s.x, acc[z + 1] = s.y;
-                        if (z + 2 < TB_Z) l = __fadd2_rn(l, dl2);
                     }
                 } else {
 #pragma unroll
