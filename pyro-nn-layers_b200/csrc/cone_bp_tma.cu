@@ -57,6 +57,7 @@ namespace {
 
 constexpr int TB_X = 32;
 constexpr int TB_Y = 8;
+constexpr long long TALL_MIN_TILES = 2048;  // 32-voxel tiles (batch included): see tall_columns
 
 // The staged box of a sinogram type: element type, row length (shifting banks
 // between rows: 64 would alias them), rows, TMA x alignment (elements) and
@@ -65,22 +66,21 @@ constexpr int TB_Y = 8;
 // 32-bit elements: element u + 1 holds taps u and u + 1, element 0 a zero tap -1
 // and tap 0.
 // TALL: columns of 32 voxels over 48 rows, which halve a thread's work per view
-// (512^3, FP16: 31.1 -> 29.1 ms).  Taken for 16-bit sinograms of volumes with many
-// voxels per detector pixel (many_voxels_per_pixel), whether the paired copy
-// exists or not, so a result does not depend on the workspace.  The others keep
-// 16 over 24: with fewer, larger tiles small volumes run out of blocks, and FP32
-// boxes leave room for 3 blocks per SM (512^3: 30.97 against 30.96 ms).
+// (512^3, FP16: 31.1 -> 28.9 ms), where many_voxels_per_pixel and tall_columns
+// say so, whether the paired copy exists or not, so a result does not depend on
+// the workspace.  The others keep 16 over 24: FP32 boxes leave room for 3 tall
+// blocks per SM (512^3: 30.97 against 30.96 ms).
 template <typename T, bool PAIRED, bool TALL>
 struct BoxLayout {
     using E = T;
     static constexpr int W = 72, ALIGN = 16 / (int)sizeof(T), OFF = 0;
     static constexpr int H = TALL ? 48 : 24, TB_Z = TALL ? 32 : 16, BP_K = TALL ? 2 : 4;
 };
-template <typename T>
-struct BoxLayout<T, true, true> {
+template <typename T, bool TALL>
+struct BoxLayout<T, true, TALL> {
     using E = unsigned;
     static constexpr int W = 68, ALIGN = 4, OFF = 1;
-    static constexpr int H = 48, TB_Z = 32, BP_K = 2;
+    static constexpr int H = TALL ? 48 : 24, TB_Z = TALL ? 32 : 16, BP_K = TALL ? 2 : 4;
 };
 
 enum ViewMode : int { MODE_SMEM = 0, MODE_GLOBAL = 1, MODE_SKIP = 2 };
@@ -164,12 +164,13 @@ __device__ __forceinline__ float interp_global(const T *__restrict__ sino, float
     return lerp_ref(lerp_first<T>(p00, p01, tx), lerp_first<T>(p10, p11, tx), ty);
 }
 
-// Resident blocks per SM the kernel is compiled for: the paired layout runs
-// best at 4 (64 registers; 3 blocks with 80: 512^3 backprojection 31.8 vs
-// 32.6 ms), the unpaired at the compiler's choice (80 registers, 3 blocks for
-// 16-bit taps: 32.5 ms, against 33.1 ms forced to 4; 0 = no minimum)
+// Resident blocks per SM the kernel is compiled for: the paired layout and tall
+// columns run best at 4 (64 registers; 3 blocks with 80: 512^3 backprojection
+// paired 31.8 vs 32.6 ms, unpaired tall, 180 views, 15.74 vs 16.61), the others at
+// the compiler's choice (80 registers, 3 blocks for 16-bit taps: 32.5 ms,
+// against 33.1 ms forced to 4; 0 = no minimum)
 #ifndef PYRONN_BP_MIN_BLOCKS
-#define PYRONN_BP_MIN_BLOCKS(paired) ((paired) ? 4 : 0)
+#define PYRONN_BP_MIN_BLOCKS(paired, tall) ((paired) || (tall) ? 4 : 0)
 #endif
 
 // Computes the metadata of one pass (warp 0 only): lane = k * 8 + corner.
@@ -245,7 +246,7 @@ __device__ __forceinline__ void pass_meta(ViewMeta *meta, const ConeBpView *__re
 }
 
 template <typename T, typename Tout, bool PAIRED, bool TALL>
-__global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED))
+__global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED, TALL))
     cone_bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, const T *__restrict__ sino, Tout *__restrict__ vol,
                        const ConeBpView *__restrict__ views, const float *__restrict__ mult, int X, int Y, int Z,
                        int W, int H, int n_proj, int geom_batch, unsigned *__restrict__ err,
@@ -537,14 +538,29 @@ inline int paired_row(int W)
     return (W + 1 + 3) / 4 * 4;
 }
 
-// whether a 16-bit sinogram takes tall columns and, given room, a paired copy:
-// the pairing pass costs about a read and two writes of the sinogram and saves a
+// whether a 16-bit sinogram takes, given room, a paired copy: the pairing pass costs about a read and two writes of the sinogram and saves a
 // shared-memory load per tap pair, worth it when a detector pixel serves many
 // voxel updates (512^3 on 1024 x 768: 171, 31.8 against 32.5 ms; 256^3 on 512^2: 64,
 // 4.26 against 4.08 ms)
 inline bool many_voxels_per_pixel(int in_dtype, const Dims3D &d)
 {
     return dtype_size(in_dtype) == 2 && (long long)d.vol_x * d.vol_y * d.vol_z >= 100LL * d.det_h * d.det_w;
+}
+
+// whether its columns are tall: where they fill their tiles as well as columns
+// of 16 do (an even number of 16-voxel tiles along z) and leave enough tiles.
+// Paired, 180 views, 16 / 32 voxels per column: 32 tiles (64^3) 0.164 / 0.297 ms,
+// 500 (160^3) 0.553 / 0.619, 1274 (208^3: 13 tiles of 16 along z) 1.172 / 1.276,
+// 1372 (224^3) 1.382 / 1.401, 1792 (256 x 224 x 256) 1.802 / 1.802, 2048 (256^3)
+// 2.007 / 1.931, 2916 (288^3) 2.823 / 2.704, 3800 (304^3: 19 along z) 3.438 /
+// 3.468, 16384 (512^3) 15.67 / 14.71.
+inline bool tall_columns(int in_dtype, const Dims3D &d)
+{
+    constexpr int TB_Z = BoxLayout<__half, false, true>::TB_Z;
+    const long long tiles = (long long)((d.vol_x + TB_X - 1) / TB_X) * ((d.vol_y + TB_Y - 1) / TB_Y) *
+                            ((d.vol_z + TB_Z - 1) / TB_Z) * d.batch;
+    const bool fills = (d.vol_z + TB_Z / 2 - 1) / (TB_Z / 2) % 2 == 0;
+    return many_voxels_per_pixel(in_dtype, d) && fills && tiles >= TALL_MIN_TILES;
 }
 
 // `pitch`: elements between the staged rows
@@ -597,13 +613,14 @@ cudaError_t launch_typed(const void *sinogram, void *volume, int in_dtype, const
                 (const Tin *)sinogram, (unsigned *)copy, d.det_w, Wp, rows);
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
-            return launch_kernel<Tin, Tout, true, true>(sinogram, copy, Wp, volume, d, views, mult, err,
-                                                        starve_last_pass, stream);
+            auto launch = tall_columns(in_dtype, d) ? launch_kernel<Tin, Tout, true, true>
+                                                    : launch_kernel<Tin, Tout, true, false>;
+            return launch(sinogram, copy, Wp, volume, d, views, mult, err, starve_last_pass, stream);
         }
     }
     auto launch_unpaired = [&](const void *staged, int pitch) {
         if constexpr (sizeof(Tin) == 2)
-            if (many_voxels_per_pixel(in_dtype, d))
+            if (tall_columns(in_dtype, d))
                 return launch_kernel<Tin, Tout, false, true>(sinogram, staged, pitch, volume, d, views, mult, err,
                                                              starve_last_pass, stream);
         return launch_kernel<Tin, Tout, false, false>(sinogram, staged, pitch, volume, d, views, mult, err,

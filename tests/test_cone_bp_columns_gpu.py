@@ -3,7 +3,10 @@ import numpy as np
 import pytest
 import torch
 
+import oracle
 import pyronn_layers as pl
+from pyronn_layers import _capi, geometry
+from conftest import rel_l2
 
 DVS = [0.9899, 0.7003, 0.6501, 0.3301]
 
@@ -32,7 +35,7 @@ def test_column_positions_do_not_drift(cuda, dtype, depth, dv):
     an ulp each."""
     dv = np.float32(dv)
     y, x, h, w = 144, 32, 38, 38
-    vol, batch = (depth, y, x), (64 if depth == 32 else 1)  # 16-bit: enough voxels and tiles for columns of 32
+    vol, batch = (depth, y, x), (128 if depth == 32 else 1)  # 16-bit: enough voxels and tiles for columns of 32
     assert depth == 16 or depth * y * x >= 100 * h * w
     P = np.array([[[1.0, 0, 0, 2.0], [0, 0, dv, 0.5], [0, 0, 0, 1.0]]], np.float32)
     rows = np.broadcast_to(np.arange(h, dtype=np.float32)[:, None], (batch, 1, h, w))
@@ -52,3 +55,39 @@ def test_drift_bound_tells_running_sums(depth):
         v = 0.5 + np.arange(0, depth, 2) * float(np.float32(dv))
         worst = max(worst, float((np.abs(_chain(np.float32(dv), 1.5, depth) - (v + 1.0)) / _bound(v)).max()))
     assert worst > 1.5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vol_shape,batch", [
+    ((64, 16, 48), 256),  # 2048 tiles of 32 voxels: tall columns
+    ((49, 16, 64), 256),  # the same, the last tile in part empty
+    ((64, 16, 48), 255),  # 2040: columns of 16
+    ((65, 16, 47), 256),  # an odd number of 16-voxel tiles along z: columns of 16
+])
+def test_column_heights(cuda, vol_shape, batch, dtype):
+    """Either column height with the paired copy and without it: the same bits,
+    and the oracle's values to FP32 rounding (1e-5, as the other paths)."""
+    geo = geometry.ConeBeam3D(vol_shape, (1.0, 1.0, 1.0), (20, 24), (5.0, 4.2), 5, 160.0, 260.0)
+    assert np.prod(vol_shape) >= 100 * 20 * 24
+    rng = np.random.Generator(np.random.PCG64(71))
+    three = rng.uniform(0.2, 1.0, (3,) + geo.detector_shape).astype(np.float32)
+    which = np.arange(batch) * 3 // batch
+    sino = torch.as_tensor(three[which]).to(device=cuda, dtype=dtype)
+    gc = pl.ops.GeometryCone(batch, cuda, *geo.args(), geo.detector_shape[0])
+    code = pl.ops.storage_code(dtype)
+    outs = []
+    for b in (batch, 0):  # with the paired copy, and the views' part alone
+        n = _capi.workspace_size("pyronn_cone_backprojection3d", b, *geo.detector_shape, *vol_shape, code, 0, 1)
+        ws = torch.empty(n, dtype=torch.uint8, device=cuda)
+        out = torch.full((batch,) + vol_shape, 7.0, device=cuda)
+        _capi.call("pyronn_cone_backprojection3d", sino.data_ptr(), out.data_ptr(), code, 0, 0, batch,
+                   *geo.detector_shape, *vol_shape, *gc.pointers(), 1, ws.data_ptr(), n,
+                   torch.cuda.current_stream().cuda_stream)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    first = [int(np.argmax(which == k)) for k in range(3)]
+    ref = oracle.cone_backprojection3d(sino[first].float().cpu().numpy(), vol_shape, *geo.args())
+    assert rel_l2(outs[0][first].cpu().numpy(), ref) < 1e-5
+    for b in range(batch):
+        assert torch.equal(outs[0][b], outs[0][first[which[b]]])
