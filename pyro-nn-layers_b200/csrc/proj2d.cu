@@ -47,7 +47,9 @@ constexpr int BP2_BLOCK_X = 32;
 constexpr int BP2_BLOCK_Y = 8;
 constexpr int BP2_CHUNK = BP2_BLOCK_X * BP2_BLOCK_Y;  // views per shared-memory table
 constexpr int BP2_VSPLIT = 4;                          // view groups of a small slice's backprojection
-constexpr long long BP2_SPLIT_MAX_PIXELS = 600000;     // threads per launch up to which view groups are used
+constexpr long long BP2_SPLIT_MAX_PIXELS = 131072;     // pixels per launch up to which view groups are used
+constexpr long long BP2_SPLIT_MAX_SHARED = 600000;     // the same, threads of several slices
+constexpr long long BP2_SHARE_MIN_PIXELS = 80000;      // pixels per launch from which a thread takes several slices
 constexpr long long BP2_NS8_MIN_PIXELS = 8000000;      // pixels per launch from which a thread takes eight slices
 
 // Two values on the packed FP32 instructions: one issue slot for both (the
@@ -609,11 +611,16 @@ __device__ __forceinline__ float fan_index_reference_steps(float cx, float cy, f
 // summing part v of every chunk's views; the groups' sums are added in
 // order at the end (the results differ from one thread's in the last bits).
 // NS > 1 (slices that share their geometry): the thread's pixel in NS slices;
-// a view's detector position, weight and tap flags are computed once.
+// a view's detector position, weight and tap flags are computed once, and a
+// block whose pixels all project inside the rows leaves the flags out.  NS = 1
+// keeps flags and row pointers: a second loop and its test cost a small slice
+// more than they save (180 views: one fan slice of 128^2, 30 -> 24 us without;
+// 16 of 256^2 with a geometry each, in fan beam, 341 -> 251 us).
 template <typename T, typename Tout, bool FAN, bool NEAR_DEPTH, int VSPLIT, int NS>
 // (eight slices: up to 128 registers; held to 80 / 64 / 48 the 64-slice fan
-// batch in FP16 takes 2.89 / 3.36 / 3.82 instead of 2.77 ms)
-__global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : 0)
+// batch in FP16 takes 2.89 / 3.36 / 3.82 instead of 2.77 ms; two parallel slices:
+// 32 registers, two of 256^2 in FP32 at 180 views 41 -> 29 us)
+__global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : (NS == 2 && !FAN ? 8 : 0))
     backprojection2d_kernel(const T *__restrict__ sino, Tout *__restrict__ vol, Geom2D geo, int X, int Y, int W,
                             int n_proj, int batch, int geom_batch)
 {
@@ -656,10 +663,30 @@ __global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : 0)
     float acc[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) acc[s] = 0.0f;
-    // (offsets within a chunk are 32-bit: rows of 2^22 pixels and more go one
-    // view at a time, taps past element 2^30 - 16 count as outside)
-    const int chunk = W < (1 << 22) ? BP2_CHUNK : 1;
-    const unsigned Wt = min(W, (1 << 30) - 16);
+    // the pixel's detector position in the view of constants q and its weight
+    auto position = [&](const float4 &q, float &w) {
+        w = 1.0f;
+        if (!FAN) return fmaf(cx, q.x, fmaf(cy, q.y, -sdo));  // (<c, d> - origin) / spacing, :51
+        // intersectLines2D(pixel, source, centre, centre + det) of
+        // fan_backprojector_2D_CudaKernel.cu.cc:52-57 in closed form:
+        // s = SDD |r|^2 <c, d> / (<c, r> + SID |r|^2), weight 1 / |c - src|^2
+        const float cd = fmaf(cy, q.x, -cx * q.y);
+        const float cr = fmaf(cx, q.x, cy * q.y);
+        const float den = cr + q.z;  // <c - src, r>: the pixel's depth from the source
+        float sidx = fmaf(q.w * cd, fast_rcp(den), -sdo);
+        // within 1e-2 mm of the source's depth, the reference's FP32 steps decide
+        if (NEAR_DEPTH && fabsf(den) < 1.0e-2f)
+            sidx = fan_index_reference_steps(cx, cy, q.x, q.y, sid, sdd, dorg, ds);
+        const float ex = fmaf(q.x, sid, cx), ey = fmaf(q.y, sid, cy);
+        w = fast_rcp(fmaf(ex, ex, ey * ey));
+        return sidx;
+    };
+    // detector positions of pixels inside the field stay far below 2^22;
+    // a pixel whose position is larger misses the row either way
+    auto clamped = [&](float sidx) { return fminf(fmaxf(sidx, -4.0f), (float)W + 4.0f); };
+    // (offsets within a chunk are 32-bit: shared rows of 2^22 pixels and more
+    // go one view at a time, taps past element 2^30 - 16 count as outside)
+    const int chunk = NS == 1 || W < (1 << 22) ? BP2_CHUNK : 1;
     for (int n0 = 0; n0 < n_proj; n0 += chunk) {
         const int cnt = min(chunk, n_proj - n0);
         __syncthreads();  // the previous chunk's constants are no longer read
@@ -679,59 +706,60 @@ __global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : 0)
             // (the detector position is monotonic along any line of pixels at
             // positive depth): all of them between the row's first and last
             // tap, with half a pixel of slack, need no tap flags
+            if (NS > 1) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float px = (float)((c & 1) ? min(i0 + BP2_BLOCK_X, X) - 1 : i0) * sx + ox;
-                const float py = (float)((c & 2) ? min(j0 + ROWS, Y) - 1 : j0) * sy + oy;
-                float s = fmaf(px, q.x, fmaf(py, q.y, -sdo));
-                if (FAN) {
-                    const float den = fmaf(px, q.x, py * q.y) + q.z;
-                    s = fmaf(q.w * fmaf(py, q.x, -px * q.y), fast_rcp(den), -sdo);
-                    all = all && den > 0.1f;
+                for (int c = 0; c < 4; ++c) {
+                    const float px = (float)((c & 1) ? min(i0 + BP2_BLOCK_X, X) - 1 : i0) * sx + ox;
+                    const float py = (float)((c & 2) ? min(j0 + ROWS, Y) - 1 : j0) * sy + oy;
+                    float s = fmaf(px, q.x, fmaf(py, q.y, -sdo));
+                    if (FAN) {
+                        const float den = fmaf(px, q.x, py * q.y) + q.z;
+                        s = fmaf(q.w * fmaf(py, q.x, -px * q.y), fast_rcp(den), -sdo);
+                        all = all && den > 0.1f;
+                    }
+                    all = all && s >= 0.5f && s <= (float)W - 1.5f;
                 }
-                all = all && s >= 0.5f && s <= (float)W - 1.5f;
             }
         }
-        const bool inside = __syncthreads_and(all);  // for all the chunk's views
+        bool inside = false;
+        if (NS > 1)
+            inside = __syncthreads_and(all);  // for all the chunk's views
+        else
+            __syncthreads();
         if (!live) continue;
         const int kb = VSPLIT == 1 ? 0 : vg * cnt / VSPLIT, ke = VSPLIT == 1 ? cnt : (vg + 1) * cnt / VSPLIT;
-        auto add_views = [&](auto check_c) {
-            constexpr bool CHECK = decltype(check_c)::value;
-            // offsets count from 8 elements before the chunk's first row, so
-            // a row's element -1 has one too
-            const char *base[NS];
-#pragma unroll
-            for (int s = 0; s < NS; ++s)
-                base[s] = reinterpret_cast<const char *>(sino_b + s * slice + (size_t)n0 * W) - 8 * sizeof(T);
-            unsigned row = (unsigned)kb * (unsigned)W + 8u;
-#pragma unroll(NEAR_DEPTH ? 1 : (NS == 1 ? 4 : 2))
+        if constexpr (NS == 1) {
+            // one slice: row pointers and flags, four views' loads in flight
+            const T *row = sino_b + (size_t)(n0 + kb) * W;
+#pragma unroll(NEAR_DEPTH ? 1 : 4)
             for (int k = kb; k < ke; ++k, row += W) {
-                const float4 q = tab[k];
-                float sidx, w = 1.0f;
-                if (!FAN) {
-                    sidx = fmaf(cx, q.x, fmaf(cy, q.y, -sdo));  // (<c, d> - origin) / spacing, :51
-                } else {
-                    // intersectLines2D(pixel, source, centre, centre + det) of
-                    // fan_backprojector_2D_CudaKernel.cu.cc:52-57 in closed form:
-                    // s = SDD |r|^2 <c, d> / (<c, r> + SID |r|^2), weight 1 / |c - src|^2
-                    const float cd = fmaf(cy, q.x, -cx * q.y);
-                    const float cr = fmaf(cx, q.x, cy * q.y);
-                    const float den = cr + q.z;  // <c - src, r>: the pixel's depth from the source
-                    sidx = fmaf(q.w * cd, fast_rcp(den), -sdo);
-                    // within 1e-2 mm of the source's depth, the reference's FP32 steps decide
-                    if (NEAR_DEPTH && fabsf(den) < 1.0e-2f)
-                        sidx = fan_index_reference_steps(cx, cy, q.x, q.y, sid, sdd, dorg, ds);
-                    const float ex = fmaf(q.x, sid, cx), ey = fmaf(q.y, sid, cy);
-                    w = fast_rcp(fmaf(ex, ex, ey * ey));
-                }
-                // detector positions of pixels inside the field stay far below 2^22;
-                // a pixel whose position is larger misses the row either way
-                const FloorFrac ff = floor_frac(CHECK ? fminf(fmaxf(sidx, -4.0f), (float)W + 4.0f) : sidx);
-                const bool in0 = (unsigned)ff.i < Wt, in1 = (unsigned)(ff.i + 1) < Wt;
-                add_row_lerps<CHECK, NS, T>(base, (row + (unsigned)ff.i) * (unsigned)sizeof(T), in0, in1, ff.f, w, acc);
+                float w;
+                const FloorFrac ff = floor_frac(clamped(position(tab[k], w)));
+                const float2 v = row_taps<true>(row + ff.i, (unsigned)ff.i < (unsigned)W, (unsigned)(ff.i + 1) < (unsigned)W);
+                acc[0] = fmaf(std::is_same<T, float>::value ? lerp_ref(v.x, v.y, ff.f) : fmaf(ff.f, v.y, v.x), w, acc[0]);
             }
-        };
-        inside ? add_views(std::false_type{}) : add_views(std::true_type{});
+        } else {
+            auto add_views = [&](auto check_c) {
+                constexpr bool CHECK = decltype(check_c)::value;
+                // offsets count from 8 elements before the chunk's first row, so
+                // a row's element -1 has one too
+                const char *base[NS];
+#pragma unroll
+                for (int s = 0; s < NS; ++s)
+                    base[s] = reinterpret_cast<const char *>(sino_b + s * slice + (size_t)n0 * W) - 8 * sizeof(T);
+                const unsigned Wt = min(W, (1 << 30) - 16);
+                unsigned row = (unsigned)kb * (unsigned)W + 8u;
+#pragma unroll(NEAR_DEPTH ? 1 : 2)
+                for (int k = kb; k < ke; ++k, row += W) {
+                    float w;
+                    const float sidx = position(tab[k], w);
+                    const FloorFrac ff = floor_frac(CHECK ? clamped(sidx) : sidx);
+                    const bool in0 = (unsigned)ff.i < Wt, in1 = (unsigned)(ff.i + 1) < Wt;
+                    add_row_lerps<CHECK, NS, T>(base, (row + (unsigned)ff.i) * (unsigned)sizeof(T), in0, in1, ff.f, w, acc);
+                }
+            };
+            inside ? add_views(std::false_type{}) : add_views(std::true_type{});
+        }
     }
     if (VSPLIT > 1) {
         __shared__ float s_acc[VSPLIT][NS][ROWS][BP2_BLOCK_X];
@@ -870,14 +898,20 @@ cudaError_t bp_typed(const void *sinogram, void *volume, bool fan, const Dims2D 
     // 256^2, 3.1 M pixels: 0.435 ms with four, 0.497 with eight; 32 of 512^2,
     // 8.4 M: 1.74 / 1.44).
     const long long pixels = (long long)d.vol_x * d.vol_y;
-    const int ns = d.geom_batch > 1 || d.batch < 2                            ? 1
+    // Launches of few pixels need the threads: 180 views, per call, one slice per
+    // thread / several: eight 64^2 fan slices (33 k pixels) 26 / 36 us, four of 128^2
+    // (66 k) 30 / 36, two of 200^2 (80 k) 38 / 26; parallel 23 / 31, 22 / 31, 31 / 29.
+    const bool share = d.geom_batch == 1 && d.batch >= 2 && d.batch * pixels >= BP2_SHARE_MIN_PIXELS;
+    const int ns = !share                                                     ? 1
                    : d.batch >= 8 && d.batch * pixels >= BP2_NS8_MIN_PIXELS ? 8
                                                                               : best_slices(d.batch, 24, 6);
     const int groups = (d.batch + ns - 1) / ns;
     // view groups for launches of few threads (see VSPLIT; three fan slices of
     // 387 x 451, 349 k threads: 0.248 ms with, 0.272 without; four of 512^2, 262 k:
-    // 0.298 / 0.322; 16 of 512^2, 1.05 M: 0.920 / 0.855)
-    const bool split = groups * pixels <= BP2_SPLIT_MAX_PIXELS;
+    // 0.298 / 0.322; 16 of 512^2, 1.05 M: 0.920 / 0.855; one slice per thread, 180
+    // views: one parallel 512^2 slice, 262 k pixels, 57 us with, 52 without; 320^2,
+    // 102 k, 35 / 32; fan 79 / 79 and 40 / 52)
+    const bool split = groups * pixels <= (ns == 1 ? BP2_SPLIT_MAX_PIXELS : BP2_SPLIT_MAX_SHARED);
     const int rows = split ? BP2_BLOCK_Y / BP2_VSPLIT : BP2_BLOCK_Y;
     const dim3 grid((d.vol_x + BP2_BLOCK_X - 1) / BP2_BLOCK_X, (d.vol_y + rows - 1) / rows, groups);
     auto launch = [&](auto kernel) {
