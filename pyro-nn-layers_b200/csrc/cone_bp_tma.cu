@@ -66,7 +66,7 @@ constexpr long long TALL_MIN_TILES = 2048;  // 32-voxel tiles (batch included): 
 // 32-bit elements: element u + 1 holds taps u and u + 1, element 0 a zero tap -1
 // and tap 0.
 // TALL: columns of 32 voxels over 48 rows, which halve a thread's work per view
-// (512^3, FP16: 31.1 -> 28.9 ms), where many_voxels_per_pixel and tall_columns
+// (512^3, FP16, 180 views: 15.6 -> 14.3 ms), where many_voxels_per_pixel and tall_columns
 // say so, whether the paired copy exists or not, so a result does not depend on
 // the workspace.  The others keep 16 over 24: FP32 boxes leave room for 3 tall
 // blocks per SM (512^3: 30.97 against 30.96 ms).
@@ -359,19 +359,16 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED, TALL)
                 if (dlv >= 0.0f && dlv < 0.999f) {
                     // rows of voxels z and z + 1 differ by 0 or 1: the pair
                     // reads rows r, r + 1, r + 2 once (three u lerps for two
-                    // voxels instead of four) and gives each voxel its two;
-                    // floors, v lerps and sums of the pair run on the packed
-                    // FP32 instructions (one issue slot for both, at half the
-                    // rate: 512^3, FP16, 31.7 -> 31.1 ms).  Each position is one
-                    // FMA from the column base: sums of 2 dlv in their place
-                    // drift by up to 15 roundings of one sign in a column of 32
-                    // (512^3: FP16 29.05 ms with the sums, 28.89 with the FMAs;
-                    // FP32 30.9 / 31.4; 256^3, FP32, 3.77 / 3.86).
-                    // The v lerp a + t (b - a) rounds as often as lerp_ref, which
-                    // needs -t as well (30.5 ms).
+                    // voxels instead of four) and gives each voxel the same
+                    // taps, hence the same bits, as the loop below.  Floors and
+                    // fractions of the pair run on the packed FP32 instructions,
+                    // one issue slot for both at half the rate.  With the v
+                    // lerps and sums packed too, 512^3 FP16 takes 28.9 instead
+                    // of 28.0 ms and 64^3, whose few warps wait for the longer
+                    // chains, 187 instead of 171 us (180 views, FP32); nothing
+                    // packed 30.2 ms / 172 us.
                     constexpr float MAGIC = 12582912.0f;  // floor_frac's, 1.5 * 2^23
                     const float2 minus1 = make_float2(-1.0f, -1.0f);
-                    const float2 rw2p = make_float2(rw2, rw2);
 #pragma unroll
                     for (int z = 0; z < TB_Z; z += 2) {
                         const float2 l = make_float2(fmaf((float)z, dlv, lv0), fmaf((float)(z + 1), dlv, lv0));
@@ -384,10 +381,8 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED, TALL)
                         const float p0 = box_ulerp<T, PAIRED>(tile + idx, tx);
                         const float p1 = box_ulerp<T, PAIRED>(tile + idx + BW, tx);
                         const float p2 = box_ulerp<T, PAIRED>(tile + idx + 2 * BW, tx);
-                        const float2 a = make_float2(p0, up ? p1 : p0), b = make_float2(p1, up ? p2 : p1);
-                        const float2 v = __ffma2_rn(fr, __ffma2_rn(a, minus1, b), a);
-                        const float2 s = __ffma2_rn(v, rw2p, make_float2(acc[z], acc[z + 1]));
-                        acc[z] = s.x, acc[z + 1] = s.y;
+                        acc[z] = fmaf(lerp_ref(p0, p1, fr.x), rw2, acc[z]);
+                        acc[z + 1] = fmaf(lerp_ref(up ? p1 : p0, up ? p2 : p1, fr.y), rw2, acc[z + 1]);
                     }
                 } else {
 #pragma unroll
@@ -549,11 +544,12 @@ inline bool many_voxels_per_pixel(int in_dtype, const Dims3D &d)
 
 // whether its columns are tall: where they fill their tiles as well as columns
 // of 16 do (an even number of 16-voxel tiles along z) and leave enough tiles.
-// Paired, 180 views, 16 / 32 voxels per column: 32 tiles (64^3) 0.164 / 0.297 ms,
-// 500 (160^3) 0.553 / 0.619, 1274 (208^3: 13 tiles of 16 along z) 1.172 / 1.276,
-// 1372 (224^3) 1.382 / 1.401, 1792 (256 x 224 x 256) 1.802 / 1.802, 2048 (256^3)
-// 2.007 / 1.931, 2916 (288^3) 2.823 / 2.704, 3800 (304^3: 19 along z) 3.438 /
-// 3.468, 16384 (512^3) 15.67 / 14.71.
+// Paired, 180 views, 16 / 32 voxels per column: 32 tiles (64^3) 0.162 / 0.295 ms,
+// 500 (160^3) 0.547 / 0.600, 1274 (208^3: 13 tiles of 16 along z) 1.166 / 1.245,
+// 1372 (224^3) 1.372 / 1.364, 2048 (256^3) 1.991 / 1.878, 2916 (288^3) 2.805 /
+// 2.624, 16384 (512^3) 15.6 / 14.3; without the copy 0.158 / 0.352, 0.539 / 0.631,
+// 1.171 / 1.369, 1.377 / 1.479, 2.002 / 2.030, 2.837 / 2.854, 16.0 / 15.7, and
+// 9.24 / 9.81 for 528 x 384 x 384 (33 tiles along z).
 inline bool tall_columns(int in_dtype, const Dims3D &d)
 {
     constexpr int TB_Z = BoxLayout<__half, false, true>::TB_Z;

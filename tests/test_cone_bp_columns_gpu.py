@@ -13,7 +13,7 @@ DVS = [0.9899, 0.7003, 0.6501, 0.3301]
 
 def _bound(v):
     """Half an ulp of the position in the box (a row above v) and of the value."""
-    return 0.5 * np.spacing((v + 1.0).astype(np.float32)) + 0.5 * np.spacing(v.astype(np.float32))
+    return 0.5 * sum(np.spacing(x.astype(np.float32)).astype(np.float64) for x in (v + 1.0, v))
 
 
 def _chain(dv, base, depth):
@@ -25,26 +25,42 @@ def _chain(dv, base, depth):
     return np.array(out, np.float64)
 
 
+def _one_view(rows, dv, depth, cuda, dtype):
+    """The backprojection of one view whose detector row is v = 0.5 + dv z, every
+    detector row holding one value: FP64 [batch, depth, y, x]."""
+    y, x, w = 144, 32, 38
+    h = len(rows)
+    batch = 128 if depth == 32 else 1  # 16-bit: enough voxels and tiles for columns of 32
+    assert depth == 16 or depth * y * x >= 100 * h * w
+    P = np.array([[[1.0, 0, 0, 2.0], [0, 0, dv, 0.5], [0, 0, 0, 1.0]]], np.float32)
+    p = torch.as_tensor(np.broadcast_to(rows[:, None], (batch, 1, h, w)).copy()).to(device=cuda, dtype=dtype)
+    out = pl.cone_backprojection3d(p, (depth, y, x), np.zeros(3), np.ones(3), P, 1.0, 1.0, out_dtype=torch.float32)
+    return out.double().cpu().numpy()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype,depth", [(torch.float32, 16), (torch.float16, 32), (torch.bfloat16, 32)])
 @pytest.mark.parametrize("dv", DVS)
 def test_column_positions_do_not_drift(cuda, dtype, depth, dv):
-    """One view whose detector row is v = 0.5 + dv z, over a sinogram of the row
-    numbers: a voxel's value is its position.  Rounded are the position from
-    the column base (one FMA; the base itself is exact) and the v lerp, half
-    an ulp each."""
-    dv = np.float32(dv)
-    y, x, h, w = 144, 32, 38, 38
-    vol, batch = (depth, y, x), (128 if depth == 32 else 1)  # 16-bit: enough voxels and tiles for columns of 32
-    assert depth == 16 or depth * y * x >= 100 * h * w
-    P = np.array([[[1.0, 0, 0, 2.0], [0, 0, dv, 0.5], [0, 0, 0, 1.0]]], np.float32)
-    rows = np.broadcast_to(np.arange(h, dtype=np.float32)[:, None], (batch, 1, h, w))
-    p = torch.as_tensor(rows.copy()).to(device=cuda, dtype=dtype)
-    out = pl.cone_backprojection3d(p, vol, np.zeros(3), np.ones(3), P, 1.0, 1.0, out_dtype=torch.float32)
-    v = 0.5 + np.arange(depth) * float(dv)
-    bound = _bound(v)
-    got = out.double().cpu().numpy()
-    assert (np.abs(got - v[None, :, None, None]) <= bound[None, :, None, None]).all()
+    """A sinogram of the row numbers: a voxel's value is its position.  Rounded
+    are the position from the column base (one FMA; the base itself is exact)
+    and the v lerp, half an ulp each."""
+    got = _one_view(np.arange(38, dtype=np.float32), dv, depth, cuda, dtype)
+    v = 0.5 + np.arange(depth) * float(np.float32(dv))
+    assert (np.abs(got - v[None, :, None, None]) <= _bound(v)[None, :, None, None]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,depth", [(torch.float32, 16), (torch.bfloat16, 32)])
+def test_column_lerp_of_rows_far_apart(cuda, dtype, depth):
+    """Rows whose difference overflows: the v lerp is a (1 - t) + t b, finite
+    for finite taps (two roundings, after the position's)."""
+    dv, a = 0.6501, float(np.float32(2.5e38) if dtype == torch.float32 else torch.tensor(2.5e38, dtype=dtype))
+    got = _one_view(np.where(np.arange(38) % 2, -a, a).astype(np.float32), dv, depth, cuda, dtype)
+    v = 0.5 + np.arange(depth) * float(np.float32(dv))
+    t, low = v - np.floor(v), np.where(np.floor(v) % 2, -a, a)
+    bound = 2 * a * _bound(v) + 1.5 * 2.0 ** 104  # (an ulp of a)
+    assert (np.abs(got - (low * (1 - 2 * t))[None, :, None, None]) <= bound[None, :, None, None]).all()
 
 
 @pytest.mark.parametrize("depth", [16, 32])
