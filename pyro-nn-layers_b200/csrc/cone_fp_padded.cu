@@ -39,8 +39,16 @@ constexpr size_t PAD_Z_BLOCKS = 16;  // z blocks of the xy-mode padded copy, eac
 // workspace header words (after the error flag) set by classify_views_kernel
 // (FLAG_WIDE, set by detect_wide_kernel: a 16-bit input holds magnitudes
 // whose differences may not fit the storage type, so the cells keep their
-// plain form and the rays take the FP32 y and x lerps)
+// plain form and the rays take the FP32 y and x lerps, from the first such
+// element of the batch on: the word is 0 or WIDE_BASE less that element, so an
+// element's form does not depend on the ones after it)
 enum { FLAG_NEED_XY = 1, FLAG_NEED_Z = 2, FLAG_WIDE = 3 };
+constexpr unsigned WIDE_BASE = 1u << 31;
+
+__device__ __forceinline__ bool wide_element(const unsigned *flags, int b)
+{
+    return flags[FLAG_WIDE] >= WIDE_BASE - (unsigned)b;
+}
 
 __global__ void classify_views_kernel(const ConeFpView *__restrict__ views, int n, unsigned *__restrict__ flags)
 {
@@ -258,28 +266,31 @@ constexpr int CELL_PLANES = 8;
 // Sets FLAG_WIDE when a 16-bit input holds a magnitude beyond Wide16's bound:
 // the cell copy then keeps the plain cells (z0 taps at y1, not differences)
 // and the rays take FP32 y and x lerps.  One read of the volume before the
-// copy, whose cell form depends on it.
+// copy, whose cell form depends on it.  blockIdx.y: the elements from b on, of
+// n values each.
 template <typename T>
-__global__ void __launch_bounds__(256) detect_wide_kernel(const T *__restrict__ src, size_t n,
+__global__ void __launch_bounds__(256) detect_wide_kernel(const T *__restrict__ src, size_t n, int b,
                                                           unsigned *__restrict__ flags)
 {
     if (!flags[FLAG_NEED_Z]) return;
     bool wide = false;
+    src += blockIdx.y * n;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         wide |= Wide16<T>::exceeds(src[i]);
-    if (__syncthreads_or(wide) && threadIdx.x == 0) atomicOr(&flags[FLAG_WIDE], 1u);
+    if (__syncthreads_or(wide) && threadIdx.x == 0) atomicMax(&flags[FLAG_WIDE], WIDE_BASE - (unsigned)(b + blockIdx.y));
 }
 
 template <typename T>
 __global__ void __launch_bounds__(PAD_TILE *8) pad_cells_kernel(const T *__restrict__ src,
                                                                  typename Cell<T>::type *__restrict__ dst, int X,
-                                                                 int Y, int Z, int s_x, unsigned *__restrict__ flags)
+                                                                 int Y, int Z, int s_x, int b,
+                                                                 unsigned *__restrict__ flags)
 {
     if (!flags[FLAG_NEED_Z]) return;
     // [y - (yc0-1)][z - (zc0-1)][x - (xc0-1)]
     __shared__ T tile[CELL_PLANES + 1][PAD_TILE + 1][PAD_TILE + 2];
     // 16-bit inputs within range take the packed lerps' y-difference cells
-    const bool ydiff = sizeof(T) == 2 && !flags[FLAG_WIDE];
+    const bool ydiff = sizeof(T) == 2 && !wide_element(flags, b);
     const int Yc = Y + 2, Zc = Z + Cell<T>::PLANES;
     const int xc0 = blockIdx.x * PAD_TILE, yc0 = blockIdx.y * CELL_PLANES, zc0 = blockIdx.z * PAD_TILE;
     for (int rr = threadIdx.y; rr < (CELL_PLANES + 1) * (PAD_TILE + 1); rr += 8) {
@@ -511,28 +522,41 @@ __device__ __forceinline__ float march_cells(const ConeRay &ray, float step, boo
 }
 
 // The march of one z-mode ray over the cell copies of NS volumes, `stride`
-// bytes apart.
-template <typename T, bool PACKED, int NS>
+// bytes apart, volume k in packed form if packed[k] (16-bit storage): together
+// where the sample count is known and the forms are the same, else one by one.
+template <typename T, int NS>
 __device__ __forceinline__ void march_cells_multi(const ConeRay &ray, float step, bool inside,
                                                   const typename Cell<T>::type *cells, size_t stride, int Z, int s_x,
-                                                  float xmax, float ymax, float zmax, float (&pixel)[NS])
+                                                  float xmax, float ymax, float zmax, const bool (&packed)[NS],
+                                                  float (&pixel)[NS])
 {
+    constexpr bool HALF = sizeof(T) == 2;
+    auto together = [&](auto packed_c, int n) {
+        constexpr bool PACKED = decltype(packed_c)::value;
+        ConeRay r = ray;
+        if (CellSampler<T, PACKED>::Z2) r.dz *= 2.0f, r.oz *= 2.0f;
+        const MultiCellSampler<T, PACKED, NS> s{CellSampler<T, PACKED>(cells, Z + Cell<T>::PLANES, s_x), stride};
+        constexpr int U = sizeof(T) == 4 ? 2 : 4;  // samples per iteration, in 64 registers
+        march_counted_multi<U, NS>(r, n, step, s, pixel);
+    };
+    auto alone = [&](int k, bool packed_k) {
+        const auto *c = (const typename Cell<T>::type *)((const char *)cells + k * stride);
+        return HALF && packed_k ? march_cells<T, HALF>(ray, step, inside, c, Z, s_x, xmax, ymax, zmax)
+                                : march_cells<T, false>(ray, step, inside, c, Z, s_x, xmax, ymax, zmax);
+    };
     if constexpr (NS == 1) {
-        pixel[0] = march_cells<T, PACKED>(ray, step, inside, cells, Z, s_x, xmax, ymax, zmax);
+        pixel[0] = alone(0, packed[0]);
     } else {
         const int n = inside ? exact_sample_count(ray, step) : -1;
-        if (n > 0) {
-            ConeRay r = ray;
-            if (CellSampler<T, PACKED>::Z2) r.dz *= 2.0f, r.oz *= 2.0f;
-            const MultiCellSampler<T, PACKED, NS> s{CellSampler<T, PACKED>(cells, Z + Cell<T>::PLANES, s_x), stride};
-            constexpr int U = sizeof(T) == 4 ? 2 : 4;  // samples per iteration, in 64 registers
-            march_counted_multi<U, NS>(r, n, step, s, pixel);
+        if (n > 0 && packed[0] == packed[NS - 1]) {
+            if (HALF && packed[0])
+                together(std::integral_constant<bool, HALF>{}, n);
+            else
+                together(std::false_type{}, n);
         } else {
 #pragma unroll 1
             for (int k = 0; k < NS; ++k) {
-                const float v = march_cells<T, PACKED>(
-                    ray, step, inside, (const typename Cell<T>::type *)((const char *)cells + k * stride), Z, s_x, xmax,
-                    ymax, zmax);
+                const float v = alone(k, k == 0 ? packed[0] : packed[NS - 1]);
                 pixel[0] = k == 0 ? v : pixel[0];
                 pixel[NS - 1] = k == NS - 1 ? v : pixel[NS - 1];
             }
@@ -579,10 +603,10 @@ __global__ void __launch_bounds__(PB_X *PB_Y, 4)
     const bool live = u < W && v < H;
     const float step = step_ptr[g];
     // 16-bit cells take the packed lerps unless the input's range forbids them
-    const bool packed = sizeof(T) == 2 && !flags[FLAG_WIDE];
+    bool packed[NS];
     float pixel[NS];
 #pragma unroll
-    for (int k = 0; k < NS; ++k) pixel[k] = 0.0f;
+    for (int k = 0; k < NS; ++k) packed[k] = sizeof(T) == 2 && !wide_element(flags, b + k), pixel[k] = 0.0f;
     if (live && in_footprint(view, u, v)) {
         const ConeRay ray = cone_ray_setup(view, u, v, X, Y, Z, 0.0, step, spacing_ptr[g * 3 + 2],
                                            spacing_ptr[g * 3 + 1], spacing_ptr[g * 3 + 0]);
@@ -590,11 +614,7 @@ __global__ void __launch_bounds__(PB_X *PB_Y, 4)
         const float xmax = (float)X + 0.999f, ymax = (float)Y + 0.999f, zmax = (float)Z + 0.999f;
         const int Xp = X + 3, Yp = Y + 3;
         if (zmode) {
-            if (packed)
-                march_cells_multi<T, sizeof(T) == 2, NS>(ray, step, inside, cells, stride, Z, cell_sx, xmax, ymax,
-                                                         zmax, pixel);
-            else
-                march_cells_multi<T, false, NS>(ray, step, inside, cells, stride, Z, cell_sx, xmax, ymax, zmax, pixel);
+            march_cells_multi<T, NS>(ray, step, inside, cells, stride, Z, cell_sx, xmax, ymax, zmax, packed, pixel);
         } else {
             // rays mostly along x -> y-fastest copy
             const double cr0 = view.inv_ar[2] + 0.5 * (W - 1) * view.inv_ar[0] + 0.5 * (H - 1) * view.inv_ar[1];
@@ -703,16 +723,15 @@ cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, co
         Tin *xfast, *yfast;
         CellT *cells;
         if constexpr (sizeof(Tin) == 2) {
-            // the cells' form depends on the range of all the launch's volumes
-            const unsigned wgrid = (unsigned)std::min<size_t>((ns * n + 255) / 256, 148 * 8);
-            detect_wide_kernel<Tin><<<wgrid, 256, 0, stream>>>((const Tin *)volume + b * n, ns * n, flags);
+            const unsigned wgrid = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 8);
+            detect_wide_kernel<Tin><<<dim3(wgrid, ns), 256, 0, stream>>>((const Tin *)volume + b * n, n, b, flags);
         }
         for (int k = 0; k < ns; ++k) {
             const Tin *src = (const Tin *)volume + (b + k) * n;
             copies(k, xfast, yfast, cells);
             pad_volume_kernel<Tin><<<pgrid, pblock, 0, stream>>>(src, xfast, yfast, d.vol_x, d.vol_y, d.vol_z, flags);
             pad_cells_kernel<Tin><<<cgrid, pblock, 0, stream>>>(src, cells, d.vol_x, d.vol_y, d.vol_z, (int)cell_sx,
-                                                                 flags);
+                                                                 b + k, flags);
         }
         copies(0, xfast, yfast, cells);
         auto launch = [&](auto kernel) {
