@@ -177,12 +177,20 @@ PYRONN_API int pyronn_fan_backprojection2d(const void *sinogram, void *volume, i
  * ------------------------------------------------------------------------- */
 /* Workspace bytes a pyronn_cone_projection3d call with these arguments needs
  * (prepared geometry; for hardware_interp = 0 also a copy of one volume as
- * trilinear cells -- the 8 taps of each cell together -- and two zero-padded
- * copies for views whose detector v axis does not run along z, all in the
- * input dtype). */
+ * trilinear cells, 16 bytes each -- the 8 taps of a cell together in 16-bit
+ * types, the four of one z in FP32, for which twice the bytes are asked -- and
+ * two zero-padded copies for views whose detector v axis does not run along z,
+ * in the input dtype). */
 PYRONN_API size_t pyronn_cone_projection3d_workspace_size(int batch, int vol_z, int vol_y, int vol_x, int n_proj,
                                                           int det_h, int det_w, int in_dtype, int hardware_interp,
                                                           int geom_batch);
+/* The same with room for a second batch element's copies: given this size, elements
+ * that share their geometry (geom_batch 1) are projected two at a time, their
+ * rays' set-up and sample positions computed once, the same results.  Equal to
+ * the query above where that does not apply. */
+PYRONN_API size_t pyronn_cone_projection3d_batched_workspace_size(int batch, int vol_z, int vol_y, int vol_x,
+                                                                  int n_proj, int det_h, int det_w, int in_dtype,
+                                                                  int hardware_interp, int geom_batch);
 
 PYRONN_API int pyronn_cone_projection3d(const void *volume, void *sinogram, int in_dtype, int out_dtype, int hardware_interp,
                              int batch, int vol_z, int vol_y, int vol_x,
@@ -201,19 +209,13 @@ PYRONN_API int pyronn_cone_projection3d(const void *volume, void *sinogram, int 
  *   step_size is accepted and unused, as in the reference.
  * ------------------------------------------------------------------------- */
 /* Workspace bytes for a pyronn_cone_backprojection3d call with these
- * arguments: the per-view geometry and, for a 16-bit sinogram on the software
- * path with at least 100 voxels per detector pixel, a paired copy of the
- * sinogram (tap u and tap u + 1 in one 32-bit element; one shared-memory load
- * per lerp, the same results).  A workspace
- * of the per-view part alone -- this size with batch = 0 -- is accepted: the
- * call then stages the sinogram itself. */
-/* The forward's workspace with room for a second batch element's copies: given
- * this size, elements that share their geometry (geom_batch 1) are projected two
- * at a time, their rays' set-up and sample positions computed once.  Equal to
- * the query above where that does not apply. */
-PYRONN_API size_t pyronn_cone_projection3d_batched_workspace_size(int batch, int vol_z, int vol_y, int vol_x,
-                                                                  int n_proj, int det_h, int det_w, int in_dtype,
-                                                                  int hardware_interp, int geom_batch);
+ * arguments: the per-view geometry and, on the software path, a copy of the
+ * sinogram: for 16-bit types with at least 100 voxels per detector pixel a
+ * paired one (tap u and tap u + 1 in one 32-bit element; one shared-memory load
+ * per lerp, the same results), else, where detector rows are no multiple of 16
+ * bytes, one at such a pitch.  A workspace of the per-view part alone -- this
+ * size with batch = 0 -- is accepted: the call then stages the sinogram itself,
+ * or, where its rows or its base are off 16 bytes, gathers from it directly. */
 PYRONN_API size_t pyronn_cone_backprojection3d_workspace_size(int batch, int n_proj, int det_h, int det_w, int vol_z,
                                                               int vol_y, int vol_x, int in_dtype,
                                                               int hardware_interp, int geom_batch);

@@ -324,7 +324,8 @@ size_t pyronn_cone_projection3d_batched_workspace_size(int batch, int vol_z, int
                                                                in_dtype, hardware_interp, geom_batch);
     const Dims3D d{batch, vol_z, vol_y, vol_x, n_proj, det_h, det_w, geom_batch};
     if (one == 0 || batch < 2 || geom_batch != 1 || hardware_interp || !cone_fp_padded_supported(d, in_dtype)) return one;
-    return one + align_up(cone_fp_padded_scratch_bytes(vol_z, vol_y, vol_x, in_dtype), 256);
+    return one + align_up(cone_fp_padded_pair_bytes(vol_z, vol_y, vol_x, in_dtype), 256) -
+           align_up(cone_fp_padded_scratch_bytes(vol_z, vol_y, vol_x, in_dtype), 256);
 }
 
 size_t pyronn_cone_backprojection3d_workspace_size(int batch, int n_proj, int det_h, int det_w, int vol_z, int vol_y,

@@ -569,8 +569,8 @@ __device__ __forceinline__ void march_cells_multi(const ConeRay &ray, float step
 // consecutive, cone_ray.cuh).  z mode: a warp is 32 consecutive v at one u, and the
 // block's 8 x 32 results go through shared memory so the sinogram rows are
 // written 8 pixels at a time; xy mode: a warp is 32 consecutive u.
-// NS = 2: batch elements b and b + 1, which share their geometry, their copies
-// `stride` bytes apart; a ray's set-up and sample positions (about 22 of the 38
+// NS = 2: batch elements b and b + 1, which share their geometry, their padded
+// copies `stride` and their cells `cell_stride` bytes apart; a ray's set-up and sample positions (about 22 of the 38
 // instructions of a sample at 128^3) are computed once.  Four volumes of 128^3,
 // 180 views of 256^2: FP32 7.22 -> 6.34 ms (the L1's lines bound it then), FP16
 // 5.98 -> 4.34; two of 181 x 203 x 219, 271 views of 287 x 347, BF16 11.8 -> 8.2.
@@ -580,8 +580,8 @@ template <typename T, typename Tout, int NS>
 // 32 resident warps hide the cell loads better than 24 with 80 registers)
 __global__ void __launch_bounds__(PB_X *PB_Y, 4)
     cone_fp_padded_kernel(const T *__restrict__ xfast, const T *__restrict__ yfast,
-                          const typename Cell<T>::type *__restrict__ cells, size_t stride, Tout *__restrict__ sino,
-                          const ConeFpView *__restrict__ views, const float *__restrict__ step_ptr,
+                          const typename Cell<T>::type *__restrict__ cells, size_t stride, size_t cell_stride,
+                          Tout *__restrict__ sino, const ConeFpView *__restrict__ views, const float *__restrict__ step_ptr,
                           const float *__restrict__ spacing_ptr, int X, int Y, int Z, int cell_sx, int W, int H,
                           int n_proj, int geom_batch, int b, const unsigned *__restrict__ flags)
 {
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(PB_X *PB_Y, 4)
         const float xmax = (float)X + 0.999f, ymax = (float)Y + 0.999f, zmax = (float)Z + 0.999f;
         const int Xp = X + 3, Yp = Y + 3;
         if (zmode) {
-            march_cells_multi<T, NS>(ray, step, inside, cells, stride, Z, cell_sx, xmax, ymax, zmax, packed, pixel);
+            march_cells_multi<T, NS>(ray, step, inside, cells, cell_stride, Z, cell_sx, xmax, ymax, zmax, packed, pixel);
         } else {
             // rays mostly along x -> y-fastest copy
             const double cr0 = view.inv_ar[2] + 0.5 * (W - 1) * view.inv_ar[0] + 0.5 * (H - 1) * view.inv_ar[1];
@@ -691,6 +691,24 @@ long long cell_x_pitch(int vol_x, int vol_y, int vol_z, size_t elem)
     return 0;
 }
 
+// The bytes of the scratch's sections: x- and y-fastest padded copies and the
+// cells of one element; those of a second, whose cells follow the first's and
+// whose padded copies come last.
+struct CopySections {
+    size_t padded, cells, single;
+    CopySections(int vol_z, int vol_y, int vol_x, size_t elem)
+    {
+        padded = section_bytes((size_t)(vol_x + 3) * (vol_y + 3) * (vol_z + 3) * elem);
+        cells = section_bytes((size_t)(vol_x + 2) * (size_t)cell_x_pitch(vol_x, vol_y, vol_z, elem) * 16);
+        // (the single query's answer is eight taps per cell for every type;
+        // FP32 cells, of four taps, use about half of it, a second element's
+        // the rest)
+        single = 2 * padded + std::max(cells, section_bytes((size_t)(vol_x + 2) * (vol_y + 2) * (vol_z + 2) * 8 * elem));
+    }
+    size_t second() const { return std::max(single, 2 * padded + 2 * cells); }
+    size_t pair() const { return second() + 2 * padded; }
+};
+
 template <typename Tin, typename Tout>
 cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, const ConeFpView *views,
                          const float *step, const float *spacing, void *scratch, bool pairs, unsigned *flags,
@@ -701,9 +719,7 @@ cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, co
     const size_t Xc = d.vol_x + 2, Yc = d.vol_y + 2, Zc = d.vol_z + Cell<Tin>::PLANES;
     const long long cell_sx = cell_x_pitch(d.vol_x, d.vol_y, d.vol_z, sizeof(Tin));
     if (cell_sx <= 0) return cudaErrorInvalidValue;
-    const size_t stride = section_bytes(cone_fp_padded_scratch_bytes(d.vol_z, d.vol_y, d.vol_x,
-                                                                     sizeof(Tin) == 4 ? PYRONN_FLOAT32 : PYRONN_FLOAT16));
-    const size_t padded = section_bytes(Xp * Yp * Zp * sizeof(Tin));
+    const CopySections sec(d.vol_z, d.vol_y, d.vol_x, sizeof(Tin));
     const int nviews = d.geom_batch * d.n_proj;
     classify_views_kernel<<<(nviews + 127) / 128, 128, 0, stream>>>(views, nviews, flags);
     const dim3 pblock(PAD_TILE, 8);
@@ -717,8 +733,9 @@ cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, co
     for (int b = 0; b < d.batch;) {
         const int ns = pairs && d.geom_batch == 1 && b + 1 < d.batch ? 2 : 1;
         auto copies = [&](int k, Tin *&xfast, Tin *&yfast, CellT *&cells) {
-            char *base = (char *)scratch + k * stride;
-            xfast = (Tin *)base, yfast = (Tin *)(base + padded), cells = (CellT *)(base + 2 * padded);
+            char *base = (char *)scratch + k * sec.second();
+            xfast = (Tin *)base, yfast = (Tin *)(base + sec.padded);
+            cells = (CellT *)((char *)scratch + 2 * sec.padded + k * sec.cells);
         };
         Tin *xfast, *yfast;
         CellT *cells;
@@ -735,8 +752,8 @@ cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, co
         }
         copies(0, xfast, yfast, cells);
         auto launch = [&](auto kernel) {
-            kernel<<<grid, block, 0, stream>>>(xfast, yfast, cells, stride, (Tout *)sinogram, views, step, spacing,
-                                               d.vol_x, d.vol_y, d.vol_z, (int)cell_sx, d.det_w, d.det_h, d.n_proj,
+            kernel<<<grid, block, 0, stream>>>(xfast, yfast, cells, sec.second(), sec.cells, (Tout *)sinogram, views,
+                                               step, spacing, d.vol_x, d.vol_y, d.vol_z, (int)cell_sx, d.det_w, d.det_h, d.n_proj,
                                                d.geom_batch, b, flags);
         };
         ns == 2 ? launch(cone_fp_padded_kernel<Tin, Tout, 2>) : launch(cone_fp_padded_kernel<Tin, Tout, 1>);
@@ -751,13 +768,12 @@ cudaError_t launch_typed(const void *volume, void *sinogram, const Dims3D &d, co
 
 size_t cone_fp_padded_scratch_bytes(int vol_z, int vol_y, int vol_x, int in_dtype)
 {
-    const size_t e = dtype_size(in_dtype);
-    const size_t padded = (size_t)(vol_x + 3) * (vol_y + 3) * (vol_z + 3);
-    const size_t cells = (size_t)(vol_x + 2) * (size_t)cell_x_pitch(vol_x, vol_y, vol_z, e);
-    // (the query's answer is eight taps per cell for every type; FP32 cells,
-    // of four taps, use about half of it)
-    const size_t taps8 = (size_t)(vol_x + 2) * (vol_y + 2) * (vol_z + 2) * 8 * e;
-    return 2 * section_bytes(padded * e) + section_bytes(std::max(cells * 16, taps8));
+    return CopySections(vol_z, vol_y, vol_x, dtype_size(in_dtype)).single;
+}
+
+size_t cone_fp_padded_pair_bytes(int vol_z, int vol_y, int vol_x, int in_dtype)
+{
+    return CopySections(vol_z, vol_y, vol_x, dtype_size(in_dtype)).pair();
 }
 
 bool cone_fp_padded_supported(const Dims3D &d, int in_dtype)

@@ -64,10 +64,12 @@ cudaError_t launch_cone_bp(const void *sinogram, void *volume, int in_dtype, int
 
 // software forward projector over padded, view-oriented copies (cone_fp_padded.cu)
 size_t cone_fp_padded_scratch_bytes(int vol_z, int vol_y, int vol_x, int in_dtype);
+// the same with a second batch element's copies
+size_t cone_fp_padded_pair_bytes(int vol_z, int vol_y, int vol_x, int in_dtype);
 bool cone_fp_padded_supported(const Dims3D &d, int in_dtype);
 // flags: zeroed header words of the workspace (the kernel records which copies it needs)
-// pairs: scratch holds two elements' copies (each 256-byte aligned), and
-// elements of shared geometry go two at a time
+// pairs: scratch is of cone_fp_padded_pair_bytes, and elements of shared
+// geometry go two at a time
 cudaError_t launch_cone_fp_padded(const void *volume, void *sinogram, int in_dtype, int out_dtype, const Dims3D &d,
                                   const ConeFpView *views, const float *step, const float *spacing, void *scratch,
                                   bool pairs, unsigned *flags, cudaStream_t stream);
