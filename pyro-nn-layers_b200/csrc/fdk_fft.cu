@@ -24,8 +24,8 @@
 // difference, over all outputs, while half of the Ram-Lak taps are zero and
 // leave the outputs they do not join to such a pixel as they are.
 //
-// The transform: N = 16 * 16 * R3, decimation in frequency forward (radices 16,
-// 16, R3, results in digit-reversed order), the product, and decimation in time
+// The transform: N = 16 * 16 * R3 (R3 = 1 for rows of up to 128 pixels), decimation
+// in frequency forward (radices 16, 16, R3, results in digit-reversed order), the product, and decimation in time
 // back, so no reordering pass exists.  A thread holds 16 complex values, and the
 // passes exchange them through shared memory (one complex of padding per 16:
 // every access of a half warp falls on 32 banks).  What bounds it: the
@@ -79,7 +79,8 @@ template <bool INV, int R>
 __device__ __forceinline__ void dft(float2 *x)
 {
     constexpr float C1 = 0.92387953251128674f, S1 = 0.38268343236508977f, H = 0.70710678118654752f;
-    if constexpr (R == 2) {
+    if constexpr (R == 1) {
+    } else if constexpr (R == 2) {
         const float2 a = x[0];
         x[0] = cadd(a, x[1]);
         x[1] = csub(a, x[1]);
@@ -135,6 +136,9 @@ struct Plan {
     static constexpr int N = 256 * R3, M = N / 16;      // points; threads per row pair
     static constexpr int PAIRS = FFT_THREADS / M;        // row pairs in flight per block
     static constexpr int PN = pad16(N);                  // padded points
+    // the group's lanes of a warp (half a warp for M = 16), and its parts of 32
+    static constexpr int LANES = M < 32 ? M : 32, PARTS = M / LANES;
+    __device__ static unsigned lane_mask(int lane) { return LANES == 32 ? 0xffffffffu : 0xffffu << (lane & 16); }
     // shared memory: the pairs' points, the kernel's spectrum, the twiddles
     // w_N^(t q) [q][t] and w_M^(t2 q) [q][t2], q = 1 .. 15
     static constexpr size_t SMEM = sizeof(float2) * ((size_t)PAIRS * PN + PN + 15 * M + 15 * R3);
@@ -158,6 +162,7 @@ __device__ __forceinline__ void forward(float2 (&x)[16], float2 *buf, const floa
 #pragma unroll
     for (int k = 0; k < 16; ++k) x[k] = buf[pad16(base + k * R3)];
     dft<false, 16>(x);
+    if (R3 == 1) return;  // (the sixteen points are the thread's)
     buf[pad16(base)] = x[0];
 #pragma unroll
     for (int q = 1; q < 16; ++q) {
@@ -177,17 +182,19 @@ template <int R3>
 __device__ __forceinline__ void inverse(float2 (&x)[16], float2 *buf, const float2 *tw1, const float2 *tw2, int t)
 {
     constexpr int M = Plan<R3>::M;
-#pragma unroll
-    for (int s = 0; s < 16 / R3; ++s) dft<true, R3>(x + s * R3);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) buf[17 * t + k] = x[k];
-    __syncthreads();
     const int t2 = t % R3, base = (t / R3) * M + t2;
-    x[0] = buf[pad16(base)];
+    if (R3 > 1) {
 #pragma unroll
-    for (int q = 1; q < 16; ++q) {
-        const float2 w = tw2[(q - 1) * R3 + t2];
-        x[q] = cmul<true>(buf[pad16(base + q * R3)], w.x, w.y);
+        for (int s = 0; s < 16 / R3; ++s) dft<true, R3>(x + s * R3);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) buf[17 * t + k] = x[k];
+        __syncthreads();
+        x[0] = buf[pad16(base)];
+#pragma unroll
+        for (int q = 1; q < 16; ++q) {
+            const float2 w = tw2[(q - 1) * R3 + t2];
+            x[q] = cmul<true>(buf[pad16(base + q * R3)], w.x, w.y);
+        }
     }
     dft<true, 16>(x);
 #pragma unroll
@@ -229,7 +236,7 @@ __device__ __noinline__ void direct_rows(const Tin *in, Tout *out, long long fir
                                          int weight_output, int nan_rows, float2 *buf, unsigned *scratch)
 {
     using P = Plan<R3>;
-    constexpr int M = P::M, WARPS = M / 32;
+    constexpr int M = P::M;
     const int tid = threadIdx.x, grp = tid / M, t = tid % M;
     float *g = reinterpret_cast<float *>(buf), *taps = g + P::N;  // W <= N / 2 of each; buf is 2 N floats and more
     for (int r = 0; r < 2; ++r) {
@@ -245,12 +252,12 @@ __device__ __noinline__ void direct_rows(const Tin *in, Tout *out, long long fir
                 g[j] = x;
                 taps[j] = fdk_tap(kind, j, du);
             }
-        const bool warp_nonfinite = __any_sync(0xffffffffu, nonfinite);
-        if ((tid & 31) == 0) scratch[tid / 32] = warp_nonfinite;
+        const bool any = __any_sync(P::lane_mask(tid & 31), nonfinite);
+        if (tid % P::LANES == 0) scratch[tid / P::LANES] = any;
         __syncthreads();  // the row is read completely before it is written
         if (bad) {
             bool all_nan = false;
-            for (int w = 0; w < WARPS; ++w) all_nan |= nan_rows && scratch[grp * WARPS + w];
+            for (int w = 0; w < P::PARTS; ++w) all_nan |= nan_rows && scratch[grp * P::PARTS + w];
             for (int j = t; j < W; j += M) {
                 float q = 0.0f;
                 if (kind == PYRONN_FILTER_RAM_LAK) {  // odd offsets and the centre
@@ -276,9 +283,9 @@ __global__ void __launch_bounds__(FFT_THREADS, FFT_BLOCKS)
                           float cv, float cu, int kind, int weight_output, int nan_rows)
 {
     using P = Plan<R3>;
-    constexpr int M = P::M, WARPS = M / 32;
+    constexpr int M = P::M, LANES = P::LANES;
     extern __shared__ __align__(16) float2 fft_smem[];
-    __shared__ unsigned peak[2][FFT_THREADS / 32];
+    __shared__ unsigned peak[2][FFT_THREADS / LANES];
     float2 *spectrum = fft_smem + P::PAIRS * P::PN, *tw1 = spectrum + P::PN, *tw2 = tw1 + 15 * M;
     const int tid = threadIdx.x, grp = tid / M, t = tid % M, lane = tid & 31;
     float2 *buf = fft_smem + grp * P::PN;
@@ -345,14 +352,14 @@ __global__ void __launch_bounds__(FFT_THREADS, FFT_BLOCKS)
             pa = max(pa, __float_as_uint(x[8].x) & 0x7fffffffu);
             pb = max(pb, __float_as_uint(x[8].y) & 0x7fffffffu);
         }
-        pa = __reduce_max_sync(0xffffffffu, pa);
-        pb = __reduce_max_sync(0xffffffffu, pb);
-        if (lane == 0) peak[0][tid / 32] = pa, peak[1][tid / 32] = pb;
+        pa = __reduce_max_sync(P::lane_mask(lane), pa);
+        pb = __reduce_max_sync(P::lane_mask(lane), pb);
+        if (lane % LANES == 0) peak[0][tid / LANES] = pa, peak[1][tid / LANES] = pb;
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) {
-            pa = max(pa, peak[0][grp * WARPS + w]);
-            pb = max(pb, peak[1][grp * WARPS + w]);
+        for (int w = 0; w < P::PARTS; ++w) {
+            pa = max(pa, peak[0][grp * P::PARTS + w]);
+            pb = max(pb, peak[1][grp * P::PARTS + w]);
         }
         // powers of two that bring the largest difference into [1, 2)
         const unsigned ea = pa >> 23, eb = pb >> 23;  // 0: zero (or flushed)
@@ -428,7 +435,8 @@ cudaError_t launch_fdk_filter_fft(const void *in, void *out, int in_dtype, int o
     return dispatch_dtypes(in_dtype, out_dtype, [&](auto tin, auto tout) -> cudaError_t {
         using Tin = typename decltype(tin)::type;
         using Tout = typename decltype(tout)::type;
-        auto launch = W <= 256    ? launch_plan<Tin, Tout, 2>
+        auto launch = W <= 128    ? launch_plan<Tin, Tout, 1>
+                      : W <= 256  ? launch_plan<Tin, Tout, 2>
                       : W <= 512  ? launch_plan<Tin, Tout, 4>
                       : W <= 1024 ? launch_plan<Tin, Tout, 8>
                                   : launch_plan<Tin, Tout, 16>;

@@ -48,7 +48,7 @@ def _rows(width, dtype):
 
 @pytest.mark.parametrize("kind", [0, 1])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("width", [37, 256, 300, 511, 1025, 2048, 2049])
+@pytest.mark.parametrize("width", [37, 128, 129, 256, 300, 511, 1025, 2048, 2049])
 @pytest.mark.parametrize("in_place", [False, True])
 def test_filter_rows_out_of_range(cuda, width, dtype, kind, in_place):
     if in_place and dtype != torch.float32:
@@ -74,3 +74,21 @@ def test_filter_rows_out_of_range(cuda, width, dtype, kind, in_place):
     for r in (0, 5):
         assert rel_l2(got[r], ref[r]) < 1e-5
     assert (got[6] == 0).all()
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("rows", [1, 2, 31, 33, 700])
+@pytest.mark.parametrize("width", [1, 2, 63, 127, 128, 129])
+def test_filter_short_rows(cuda, width, rows, kind):
+    """Rows about the width of the shortest transform, two groups of threads to
+    a warp: each row to 1e-5 (as test_fbp_gpu.py), whatever its neighbours."""
+    p = np.random.Generator(np.random.PCG64(width + rows)).uniform(0.2, 1.0, (rows, width)).astype(np.float32)
+    p[1::3] *= np.float32(1e-7)
+    x = torch.as_tensor(p, device=cuda)
+    out = torch.empty_like(x)
+    _capi.call("pyronn_fdk_filter", x.data_ptr(), out.data_ptr(), 0, 0, 1, 1, rows, width, SDD, DV, DU, (rows - 1) / 2,
+               (width - 1) / 2, kind, 0, torch.cuda.current_stream().cuda_stream)
+    ref, _ = _direct(p, kind)
+    got = out.double().cpu().numpy()
+    for r in range(rows):
+        assert rel_l2(got[r], ref[r]) < 1e-5
