@@ -85,6 +85,7 @@ size_t align_up(size_t n, size_t a)
 // every cone workspace starts with a header whose first word is the device
 // error flag of the call (pyronn::DeviceError), cleared at the start of the call
 constexpr size_t WS_HEADER = 256;
+constexpr int WS_DIRECT_WORD = 4;  // backprojection: set by the device when the direct kernel does the work
 
 bool valid_dtype(int dtype)
 {
@@ -445,11 +446,17 @@ int pyronn_cone_backprojection3d(const void *sinogram, void *volume, int in_dtyp
     if (!hardware_interp) {
         const size_t cb = cone_bp_tma_copy_bytes(in_dtype, d);
         void *copy = (cb > 0 && workspace_bytes >= need + cb) ? (char *)workspace + need : nullptr;
-        if (cone_bp_tma_supported(sinogram, in_dtype, d, copy != nullptr))
+        if (cone_bp_tma_supported(sinogram, in_dtype, d, copy != nullptr)) {
+            // rows TMA cannot address: the device says whether a copy pays
+            unsigned *direct = copy && !cone_bp_tma_aligned(sinogram, in_dtype, d) ? err + WS_DIRECT_WORD : nullptr;
             e = launch_cone_bp_tma(sinogram, volume, in_dtype, out_dtype, d, views, projection_multiplier, err, copy,
-                                   s);
-        else
+                                   direct, s);
+            if (e == cudaSuccess && direct)
+                e = launch_cone_bp(sinogram, volume, in_dtype, out_dtype, d, -1, views, projection_multiplier, 0, s,
+                                   direct);
+        } else {
             e = launch_cone_bp(sinogram, volume, in_dtype, out_dtype, d, -1, views, projection_multiplier, 0, s);
+        }
         if (e != cudaSuccess) return cuda_fail(e, name);
         return ok();
     }

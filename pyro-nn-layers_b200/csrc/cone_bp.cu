@@ -56,8 +56,9 @@ template <typename T, typename Tout, bool HW>
 __global__ void __launch_bounds__(BP_BLOCK_X *BP_BLOCK_Y)
     cone_bp_kernel(const T *__restrict__ sino, Tout *__restrict__ vol, const ConeBpView *__restrict__ views,
                    const float *__restrict__ mult, int X, int Y, int Z, int W, int H, int n_proj, int geom_batch,
-                   int batch_begin, cudaTextureObject_t tex)
+                   int batch_begin, cudaTextureObject_t tex, const unsigned *__restrict__ only_if)
 {
+    if (only_if && !*only_if) return;
     const int i = blockIdx.x * BP_BLOCK_X + threadIdx.x;
     const int j = blockIdx.y * BP_BLOCK_Y + threadIdx.y;
     const int zblocks = (Z + BP_ZB - 1) / BP_ZB;
@@ -108,7 +109,8 @@ __global__ void __launch_bounds__(BP_BLOCK_X *BP_BLOCK_Y)
 
 template <typename Tin, typename Tout>
 cudaError_t launch_typed(const void *sinogram, void *volume, const Dims3D &d, int batch_begin, int batch_count,
-                         const ConeBpView *views, const float *mult, cudaTextureObject_t tex, cudaStream_t stream)
+                         const ConeBpView *views, const float *mult, cudaTextureObject_t tex, const unsigned *only_if,
+                         cudaStream_t stream)
 {
     const dim3 block(BP_BLOCK_X, BP_BLOCK_Y, 1);
     const int zblocks = (d.vol_z + BP_ZB - 1) / BP_ZB;
@@ -120,11 +122,11 @@ cudaError_t launch_typed(const void *sinogram, void *volume, const Dims3D &d, in
         if (tex)  // the texture holds the data; the input pointer is not read
             cone_bp_kernel<float, Tout, true><<<grid, block, 0, stream>>>(
                 nullptr, (Tout *)volume, views, mult, d.vol_x, d.vol_y, d.vol_z, d.det_w, d.det_h, d.n_proj,
-                d.geom_batch, batch_begin + b0, tex);
+                d.geom_batch, batch_begin + b0, tex, only_if);
         else
             cone_bp_kernel<Tin, Tout, false><<<grid, block, 0, stream>>>(
                 (const Tin *)sinogram, (Tout *)volume, views, mult, d.vol_x, d.vol_y, d.vol_z, d.det_w, d.det_h,
-                d.n_proj, d.geom_batch, batch_begin + b0, tex);
+                d.n_proj, d.geom_batch, batch_begin + b0, tex, only_if);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -135,14 +137,14 @@ cudaError_t launch_typed(const void *sinogram, void *volume, const Dims3D &d, in
 
 cudaError_t launch_cone_bp(const void *sinogram, void *volume, int in_dtype, int out_dtype, const Dims3D &d,
                            int batch_index, const ConeBpView *views, const float *mult, cudaTextureObject_t tex,
-                           cudaStream_t stream)
+                           cudaStream_t stream, const unsigned *only_if)
 {
     const int b0 = batch_index < 0 ? 0 : batch_index;
     const int nb = batch_index < 0 ? d.batch : 1;
     return dispatch_dtypes(in_dtype, out_dtype, [&](auto tin, auto tout) {
         using Tin = typename decltype(tin)::type;
         using Tout = typename decltype(tout)::type;
-        return launch_typed<Tin, Tout>(sinogram, volume, d, b0, nb, views, mult, tex, stream);
+        return launch_typed<Tin, Tout>(sinogram, volume, d, b0, nb, views, mult, tex, only_if, stream);
     });
 }
 

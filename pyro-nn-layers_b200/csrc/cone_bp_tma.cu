@@ -26,7 +26,8 @@
 // Detector rows that are no multiple of 16 bytes, which TMA cannot address,
 // are likewise copied to rows of such a pitch first (the paired copy where
 // that pays, else a plain one): 181 x 203 x 219 voxels, 271 views of 287 x 347 in
-// BF16 take 2.2 ms, the copy included, against 6.3 ms in the direct-gather kernel.
+// BF16 take 2.2 ms, the copy included, against 6.3 ms in the direct-gather kernel,
+// which keeps the scans whose boxes would not fit (route_kernel).
 //
 // Exactness: the tap indices and weights are computed exactly as the direct
 // path computes them (floor of u/w, frac), only the texel source differs.  TMA
@@ -46,6 +47,7 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -250,8 +252,9 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED, TALL)
     cone_bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, const T *__restrict__ sino, Tout *__restrict__ vol,
                        const ConeBpView *__restrict__ views, const float *__restrict__ mult, int X, int Y, int Z,
                        int W, int H, int n_proj, int geom_batch, unsigned *__restrict__ err,
-                       int starve_last_pass)
+                       int starve_last_pass, const unsigned *__restrict__ direct)
 {
+    if (direct && *direct) return;  // the direct kernel's launch
     extern __shared__ __align__(128) unsigned char dyn_smem[];
     // TMA destinations must be 128-byte aligned: round the base up (the
     // launch reserves 128 spare bytes); every tile is a multiple of 128 bytes
@@ -447,6 +450,34 @@ __global__ void __launch_bounds__(TB_X *TB_Y, PYRONN_BP_MIN_BLOCKS(PAIRED, TALL)
     }
 }
 
+// Whether rows TMA cannot address are worth a copy: only boxes that fit are
+// staged from it, and a detector of many rows per voxel (above about 1.4: 24 rows
+// under 16 voxels) overflows them; the direct kernel then does the work, which
+// the global path here does slower (128^3 voxels, 60 views of 724 x 723, FP16:
+// 526 us against 453, the copy included; 465 with this choice).  *direct is set when more than two of
+// three (tile, view) pairs with taps on the detector do not fit, of eight passes
+// spread over the views and the four tiles about the middles of the volume's
+// quadrants at its middle depth.  One block, a warp for each.
+constexpr int ROUTE_PASSES = 8, ROUTE_WARPS = 4 * ROUTE_PASSES;
+template <typename T, bool PAIRED, bool TALL>
+__global__ void __launch_bounds__(32 * ROUTE_WARPS)
+    route_kernel(const ConeBpView *__restrict__ views, int X, int Y, int Z, int W, int H, int n_proj,
+                 unsigned *__restrict__ direct)
+{
+    using L = BoxLayout<T, PAIRED, TALL>;
+    __shared__ ViewMeta meta[ROUTE_WARPS][L::BP_K];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, pass = warp / 4;
+    const int n_pass = (n_proj + L::BP_K - 1) / L::BP_K;
+    const int first = (int)((long long)pass * n_pass / ROUTE_PASSES) * L::BP_K;
+    auto tile = [](int extent, int quarter, int size) { return (int)((long long)extent * quarter / 4) / size * size; };
+    pass_meta<T, PAIRED, TALL>(meta[warp], views, first, n_proj, tile(X, warp & 1 ? 3 : 1, TB_X),
+                               tile(Y, warp & 2 ? 3 : 1, TB_Y), tile(Z, 2, L::TB_Z), W, H);
+    __syncwarp();
+    const int mode = lane < L::BP_K && first + lane < n_proj ? meta[warp][lane].mode : MODE_SKIP;
+    const int staged = __syncthreads_count(mode == MODE_SMEM), global = __syncthreads_count(mode == MODE_GLOBAL);
+    if (threadIdx.x == 0) *direct = global > 2 * staged;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -490,8 +521,10 @@ CUtensorMapDataType tma_type<__half>()
 // elements by rows (a row per blockIdx.y, strided).
 template <typename T>
 __global__ void __launch_bounds__(256)
-    pair_sinogram_kernel(const T *__restrict__ sino, unsigned *__restrict__ paired, int W, int Wp, long long rows)
+    pair_sinogram_kernel(const T *__restrict__ sino, unsigned *__restrict__ paired, int W, int Wp, long long rows,
+                         const unsigned *__restrict__ direct)
 {
+    if (direct && *direct) return;
     const int x = blockIdx.x * 256 + threadIdx.x;
     if (x >= Wp) return;
     for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
@@ -506,8 +539,10 @@ __global__ void __launch_bounds__(256)
 // a multiple of 16 bytes.  Grid as the pairing's; a thread writes 16 bytes.
 template <typename T>
 __global__ void __launch_bounds__(256)
-    pitch_sinogram_kernel(const T *__restrict__ sino, T *__restrict__ dst, int W, int Wp, long long rows)
+    pitch_sinogram_kernel(const T *__restrict__ sino, T *__restrict__ dst, int W, int Wp, long long rows,
+                          const unsigned *__restrict__ direct)
 {
+    if (direct && *direct) return;
     constexpr int N = 16 / (int)sizeof(T);
     const int x = (blockIdx.x * 256 + threadIdx.x) * N;
     if (x >= Wp) return;
@@ -563,7 +598,7 @@ inline bool tall_columns(int in_dtype, const Dims3D &d)
 template <typename Tin, typename Tout, bool PAIRED, bool TALL>
 cudaError_t launch_kernel(const void *sinogram, const void *staged, int pitch, void *volume, const Dims3D &d,
                           const ConeBpView *views, const float *mult, unsigned *err, int starve_last_pass,
-                          cudaStream_t stream)
+                          const unsigned *direct, cudaStream_t stream)
 {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
@@ -592,46 +627,48 @@ cudaError_t launch_kernel(const void *sinogram, const void *staged, int pitch, v
     if (e != cudaSuccess) return e;
     cone_bp_tma_kernel<Tin, Tout, PAIRED, TALL><<<grid, block, smem, stream>>>(
         map, (const Tin *)sinogram, (Tout *)volume, views, mult, d.vol_x, d.vol_y, d.vol_z, d.det_w, d.det_h, d.n_proj,
-        d.geom_batch, err, starve_last_pass);
+        d.geom_batch, err, starve_last_pass, direct);
     return cudaGetLastError();
 }
 
+// `direct`: with a copy, a word the device sets when the direct kernel is to do
+// the work, which is launched after this; or null.
 template <typename Tin, typename Tout>
 cudaError_t launch_typed(const void *sinogram, void *volume, int in_dtype, const Dims3D &d, const ConeBpView *views,
-                         const float *mult, unsigned *err, int starve_last_pass, void *copy, cudaStream_t stream)
+                         const float *mult, unsigned *err, int starve_last_pass, void *copy, unsigned *direct,
+                         cudaStream_t stream)
 {
     const long long rows = (long long)d.batch * d.n_proj * d.det_h;
-    const unsigned ygrid = (unsigned)(rows < 65535 ? rows : 65535);
-    if constexpr (sizeof(Tin) == 2) {
-        if (copy && many_voxels_per_pixel(in_dtype, d)) {
-            const int Wp = paired_row(d.det_w);
-            pair_sinogram_kernel<Tin><<<dim3((unsigned)((Wp + 255) / 256), ygrid), 256, 0, stream>>>(
-                (const Tin *)sinogram, (unsigned *)copy, d.det_w, Wp, rows);
-            cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return e;
-            auto launch = tall_columns(in_dtype, d) ? launch_kernel<Tin, Tout, true, true>
-                                                    : launch_kernel<Tin, Tout, true, false>;
-            return launch(sinogram, copy, Wp, volume, d, views, mult, err, starve_last_pass, stream);
+    const unsigned ygrid = (unsigned)(rows < 4096 ? rows : 4096);  // (few blocks to start where nothing is copied)
+    auto run = [&](auto paired_c, auto tall_c) -> cudaError_t {
+        constexpr bool PAIRED = decltype(paired_c)::value, TALL = decltype(tall_c)::value;
+        if (copy && direct)
+            route_kernel<Tin, PAIRED, TALL><<<1, 32 * ROUTE_WARPS, 0, stream>>>(views, d.vol_x, d.vol_y, d.vol_z,
+                                                                                d.det_w, d.det_h, d.n_proj, direct);
+        int pitch = d.det_w;
+        if constexpr (PAIRED) {
+            pitch = paired_row(d.det_w);
+            pair_sinogram_kernel<Tin><<<dim3((unsigned)((pitch + 255) / 256), ygrid), 256, 0, stream>>>(
+                (const Tin *)sinogram, (unsigned *)copy, d.det_w, pitch, rows, direct);
+        } else if (copy) {
+            pitch = pitched_row(d.det_w, sizeof(Tin));
+            const int chunks = pitch / (16 / (int)sizeof(Tin));
+            pitch_sinogram_kernel<Tin><<<dim3((unsigned)((chunks + 255) / 256), ygrid), 256, 0, stream>>>(
+                (const Tin *)sinogram, (Tin *)copy, d.det_w, pitch, rows, direct);
         }
-    }
-    auto launch_unpaired = [&](const void *staged, int pitch) {
-        if constexpr (sizeof(Tin) == 2)
-            if (tall_columns(in_dtype, d))
-                return launch_kernel<Tin, Tout, false, true>(sinogram, staged, pitch, volume, d, views, mult, err,
-                                                             starve_last_pass, stream);
-        return launch_kernel<Tin, Tout, false, false>(sinogram, staged, pitch, volume, d, views, mult, err,
-                                                      starve_last_pass, stream);
-    };
-    if (copy) {
-        const int Wp = pitched_row(d.det_w, sizeof(Tin));
-        const int chunks = Wp / (16 / (int)sizeof(Tin));
-        pitch_sinogram_kernel<Tin><<<dim3((unsigned)((chunks + 255) / 256), ygrid), 256, 0, stream>>>(
-            (const Tin *)sinogram, (Tin *)copy, d.det_w, Wp, rows);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        return launch_unpaired(copy, Wp);
+        return launch_kernel<Tin, Tout, PAIRED, TALL>(sinogram, copy ? copy : sinogram, pitch, volume, d, views, mult,
+                                                      err, starve_last_pass, direct, stream);
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    if constexpr (sizeof(Tin) == 2) {
+        const bool tall = tall_columns(in_dtype, d);
+        if (copy && many_voxels_per_pixel(in_dtype, d)) return tall ? run(yes, yes) : run(yes, no);
+        if (tall) return run(no, yes);
     }
-    return launch_unpaired(sinogram, d.det_w);
+    return run(no, no);
 }
 
 }  // namespace
@@ -639,11 +676,15 @@ cudaError_t launch_typed(const void *sinogram, void *volume, int in_dtype, const
 // The TMA path needs 16-byte aligned rows and base (the sinogram's, or a
 // copy's) and a grid that fits one launch; the caller falls back to the direct
 // kernel otherwise.
+bool cone_bp_tma_aligned(const void *sinogram, int in_dtype, const Dims3D &d)
+{
+    return (uintptr_t)sinogram % 16 == 0 && ((size_t)d.det_w * dtype_size(in_dtype)) % 16 == 0;
+}
+
 bool cone_bp_tma_supported(const void *sinogram, int in_dtype, const Dims3D &d, bool copy)
 {
-    const size_t e = dtype_size(in_dtype);
-    if (e == 0) return false;
-    if (!copy && (((uintptr_t)sinogram % 16) != 0 || ((size_t)d.det_w * e) % 16 != 0)) return false;
+    if (dtype_size(in_dtype) == 0) return false;
+    if (!copy && !cone_bp_tma_aligned(sinogram, in_dtype, d)) return false;
     constexpr int TB_Z = BoxLayout<float, false, false>::TB_Z;  // the shorter columns
     const long long zb = (d.vol_z + TB_Z - 1) / TB_Z;
     if (zb * d.batch > 65535 || (d.vol_y + TB_Y - 1) / TB_Y > 65535) return false;
@@ -670,13 +711,13 @@ size_t cone_bp_tma_copy_bytes(int in_dtype, const Dims3D &d)
 
 cudaError_t launch_cone_bp_tma(const void *sinogram, void *volume, int in_dtype, int out_dtype, const Dims3D &d,
                                const ConeBpView *views, const float *mult, unsigned *err, void *copy,
-                               cudaStream_t stream)
+                               unsigned *direct, cudaStream_t stream)
 {
     const int starve = g_starve_last_pass.load();
     return dispatch_dtypes(in_dtype, out_dtype, [&](auto tin, auto tout) {
         using Tin = typename decltype(tin)::type;
         using Tout = typename decltype(tout)::type;
-        return launch_typed<Tin, Tout>(sinogram, volume, in_dtype, d, views, mult, err, starve, copy, stream);
+        return launch_typed<Tin, Tout>(sinogram, volume, in_dtype, d, views, mult, err, starve, copy, direct, stream);
     });
 }
 

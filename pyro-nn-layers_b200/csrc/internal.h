@@ -54,13 +54,14 @@ cudaError_t launch_projection2d(const void *volume, void *sinogram, int in_dtype
 cudaError_t launch_backprojection2d(const void *sinogram, void *volume, int in_dtype, int out_dtype, bool fan,
                                     const Dims2D &d, const Geom2D &g, cudaStream_t stream);
 
-// cone (cone_fp.cu / cone_bp.cu); tex == 0 selects the software path
+// cone (cone_fp.cu / cone_bp.cu); tex == 0 selects the software path;
+// only_if: a device word, the launch does nothing where it is 0 (or null)
 cudaError_t launch_cone_fp(const void *volume, void *sinogram, int in_dtype, int out_dtype, const Dims3D &d,
                            int batch_index, const ConeFpView *views, const float *step, const float *spacing,
                            cudaTextureObject_t tex, cudaStream_t stream);
 cudaError_t launch_cone_bp(const void *sinogram, void *volume, int in_dtype, int out_dtype, const Dims3D &d,
                            int batch_index, const ConeBpView *views, const float *mult, cudaTextureObject_t tex,
-                           cudaStream_t stream);
+                           cudaStream_t stream, const unsigned *only_if = nullptr);
 
 // software forward projector over padded, view-oriented copies (cone_fp_padded.cu)
 size_t cone_fp_padded_scratch_bytes(int vol_z, int vol_y, int vol_x, int in_dtype);
@@ -100,14 +101,18 @@ cudaError_t launch_cone_scatter(const void *sinogram, float *volume, int in_dtyp
 // TMA-staged software backprojector (cone_bp_tma.cu); err = device error flag
 // (copy: a copy of cone_bp_tma_copy_bytes will be given)
 bool cone_bp_tma_supported(const void *sinogram, int in_dtype, const Dims3D &d, bool copy);
+// whether the sinogram's own rows can be staged
+bool cone_bp_tma_aligned(const void *sinogram, int in_dtype, const Dims3D &d);
 // Bytes of the copy of the sinogram the TMA backprojector stages its boxes
 // from: 32-bit tap pairs of a 16-bit sinogram where that pays (one shared-memory
 // load per lerp), rows at a 16-byte pitch where the sinogram's are none; else 0.
 size_t cone_bp_tma_copy_bytes(int in_dtype, const Dims3D &d);
-// `copy` (device, 16-byte aligned, cone_bp_tma_copy_bytes) or null.
+// `copy` (device, 16-byte aligned, cone_bp_tma_copy_bytes) or null.  `direct`, with
+// a copy: a device word that is set, and nothing else written, where launch_cone_bp
+// should do the work (given the same word, it works only then); or null.
 cudaError_t launch_cone_bp_tma(const void *sinogram, void *volume, int in_dtype, int out_dtype, const Dims3D &d,
                                const ConeBpView *views, const float *mult, unsigned *err, void *copy,
-                               cudaStream_t stream);
+                               unsigned *direct, cudaStream_t stream);
 // testing hook (pyronn_debug_starve_tma_wait): while enabled, the last pass of
 // every TMA backprojector block issues no copies and expects bytes that never
 // arrive, so its bounded wait runs out and the block reports the timeout

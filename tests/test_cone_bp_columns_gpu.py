@@ -1,4 +1,4 @@
-"""GPU tests of the cone backprojector's column loop."""
+"""Tests of the cone backprojector's column loop and of its choice of kernel."""
 import numpy as np
 import pytest
 import torch
@@ -107,3 +107,38 @@ def test_column_heights(cuda, vol_shape, batch, dtype):
     assert rel_l2(outs[0][first].cpu().numpy(), ref) < 1e-5
     for b in range(batch):
         assert torch.equal(outs[0][b], outs[0][first[which[b]]])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vol_shape,det,pitch,batch,fits", [
+    ((40, 44, 48), (61, 67), 1.3, 1, True),     # about one row per voxel
+    ((40, 44, 48), (301, 331), 0.26, 1, False),  # six: the boxes overflow
+    ((17, 9, 33), (151, 133), 0.4, 3, False),
+    ((1, 1, 1), (5, 3), 1.0, 2, False),  # the tile reaches past the detector
+])
+def test_rows_off_16_bytes(cuda, vol_shape, det, pitch, batch, fits, dtype):
+    """Rows TMA cannot address, given the copy's workspace: staged from it where
+    the boxes fit, else the direct kernel's bits; the oracle's values either
+    way, nothing written past the workspace."""
+    geo = geometry.ConeBeam3D(vol_shape, (1.0, 1.0, 1.0), det, (pitch, pitch), 9, 160.0, 260.0)
+    rng = np.random.Generator(np.random.PCG64(72))
+    sino = torch.as_tensor(rng.uniform(0.2, 1.0, (batch,) + geo.detector_shape)).to(device=cuda, dtype=dtype)
+    gc = pl.ops.GeometryCone(batch, cuda, *geo.args(), geo.detector_shape[0])
+    code = pl.ops.storage_code(dtype)
+    outs = []
+    for b in (batch, 0):
+        n = _capi.workspace_size("pyronn_cone_backprojection3d", b, *geo.detector_shape, *vol_shape, code, 0, 1)
+        ws = torch.full((n + 256,), 0xA5, dtype=torch.uint8, device=cuda)
+        out = torch.full((batch,) + vol_shape, 7.0, device=cuda)
+        _capi.call("pyronn_cone_backprojection3d", sino.data_ptr(), out.data_ptr(), code, 0, 0, batch,
+                   *geo.detector_shape, *vol_shape, *gc.pointers(), 1, ws.data_ptr(), n,
+                   torch.cuda.current_stream().cuda_stream)
+        assert bool((ws[n:] == 0xA5).all())
+        outs.append((out, ws[16:20].view(torch.int32).item()))
+    assert outs[0][1] == (0 if fits else 1) and outs[1][1] == 0
+    if not fits:
+        assert torch.equal(outs[0][0], outs[1][0])
+    ref = oracle.cone_backprojection3d(sino.float().cpu().numpy(), vol_shape, *geo.args())
+    for out, _ in outs:
+        assert rel_l2(out.cpu().numpy(), ref) < 1e-5
