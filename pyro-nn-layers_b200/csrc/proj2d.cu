@@ -612,10 +612,11 @@ __device__ __forceinline__ float fan_index_reference_steps(float cx, float cy, f
 // order at the end (the results differ from one thread's in the last bits).
 // NS > 1 (slices that share their geometry): the thread's pixel in NS slices;
 // a view's detector position, weight and tap flags are computed once, and a
-// block whose pixels all project inside the rows leaves the flags out.  NS = 1
-// keeps flags and row pointers: a second loop and its test cost a small slice
-// more than they save (180 views: one fan slice of 128^2, 30 -> 24 us without;
-// 16 of 256^2 with a geometry each, in fan beam, 341 -> 251 us).
+// block whose pixels all project inside the rows leaves the flags out.  One slice
+// of a fan or in view groups keeps flags and row pointers: a second loop and its
+// test cost it more than they save (180 views: one fan slice of 128^2, 30 -> 24 us
+// without; 16 of 256^2 with a geometry each, in fan beam, 341 -> 251 us; but one
+// parallel slice of 1024^2, 90 views, 72 us with, 92 without).
 template <typename T, typename Tout, bool FAN, bool NEAR_DEPTH, int VSPLIT, int NS>
 // (eight slices: up to 128 registers; held to 80 / 64 / 48 the 64-slice fan
 // batch in FP16 takes 2.89 / 3.36 / 3.82 instead of 2.77 ms; two parallel slices:
@@ -625,6 +626,7 @@ __global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : (NS ==
                             int n_proj, int batch, int geom_batch)
 {
     constexpr int ROWS = BP2_BLOCK_Y / VSPLIT;  // pixel rows per block
+    constexpr bool ALWAYS_FLAGS = NS == 1 && (FAN || VSPLIT > 1);
     __shared__ float4 tab[BP2_CHUNK];
     const int vg = threadIdx.y / ROWS;          // view group
     const int i0 = blockIdx.x * BP2_BLOCK_X, j0 = blockIdx.y * ROWS;
@@ -686,7 +688,7 @@ __global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : (NS ==
     auto clamped = [&](float sidx) { return fminf(fmaxf(sidx, -4.0f), (float)W + 4.0f); };
     // (offsets within a chunk are 32-bit: shared rows of 2^22 pixels and more
     // go one view at a time, taps past element 2^30 - 16 count as outside)
-    const int chunk = NS == 1 || W < (1 << 22) ? BP2_CHUNK : 1;
+    const int chunk = ALWAYS_FLAGS || W < (1 << 22) ? BP2_CHUNK : 1;
     for (int n0 = 0; n0 < n_proj; n0 += chunk) {
         const int cnt = min(chunk, n_proj - n0);
         __syncthreads();  // the previous chunk's constants are no longer read
@@ -706,7 +708,7 @@ __global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : (NS ==
             // (the detector position is monotonic along any line of pixels at
             // positive depth): all of them between the row's first and last
             // tap, with half a pixel of slack, need no tap flags
-            if (NS > 1) {
+            if (!ALWAYS_FLAGS) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float px = (float)((c & 1) ? min(i0 + BP2_BLOCK_X, X) - 1 : i0) * sx + ox;
@@ -722,13 +724,13 @@ __global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : (NS ==
             }
         }
         bool inside = false;
-        if (NS > 1)
-            inside = __syncthreads_and(all);  // for all the chunk's views
-        else
+        if (ALWAYS_FLAGS)
             __syncthreads();
+        else
+            inside = __syncthreads_and(all);  // for all the chunk's views
         if (!live) continue;
         const int kb = VSPLIT == 1 ? 0 : vg * cnt / VSPLIT, ke = VSPLIT == 1 ? cnt : (vg + 1) * cnt / VSPLIT;
-        if constexpr (NS == 1) {
+        if constexpr (ALWAYS_FLAGS) {
             // one slice: row pointers and flags, four views' loads in flight
             const T *row = sino_b + (size_t)(n0 + kb) * W;
 #pragma unroll(NEAR_DEPTH ? 1 : 4)
@@ -749,7 +751,7 @@ __global__ void __launch_bounds__(BP2_BLOCK_X *BP2_BLOCK_Y, NS == 8 ? 2 : (NS ==
                     base[s] = reinterpret_cast<const char *>(sino_b + s * slice + (size_t)n0 * W) - 8 * sizeof(T);
                 const unsigned Wt = min(W, (1 << 30) - 16);
                 unsigned row = (unsigned)kb * (unsigned)W + 8u;
-#pragma unroll(NEAR_DEPTH ? 1 : 2)
+#pragma unroll(NEAR_DEPTH ? 1 : (NS == 1 ? 4 : 2))
                 for (int k = kb; k < ke; ++k, row += W) {
                     float w;
                     const float sidx = position(tab[k], w);
