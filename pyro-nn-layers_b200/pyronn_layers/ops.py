@@ -74,20 +74,30 @@ _HOST_GEOM_CACHE: "collections.OrderedDict" = collections.OrderedDict()
 _HOST_GEOM_CACHE_SIZE = 64
 
 
+def _host_array(t) -> np.ndarray:
+    return np.ascontiguousarray(t.detach().numpy() if isinstance(t, torch.Tensor) else t, dtype=np.float32)
+
+
+def _content(a: np.ndarray) -> bytes:
+    return a.tobytes() if a.nbytes <= 4096 else hashlib.blake2b(a.data, digest_size=16).digest()
+
+
 class _HostArray:
     """A host array as float32, with its content as a key and, once it is on a
     device, the streams its copy there is recorded on."""
 
     __slots__ = ("array", "key", "streams")
 
-    def __init__(self, t):
-        a = t.detach().numpy() if isinstance(t, torch.Tensor) else t
-        self.array = a = np.ascontiguousarray(a, dtype=np.float32)
-        self.key = (a.shape, a.tobytes() if a.nbytes <= 4096 else hashlib.blake2b(a.data, digest_size=16).digest())
+    def __init__(self, array, content):
+        self.array, self.key = array, (array.shape, content)
 
 
 def _host_geometry_on_device(t, device) -> torch.Tensor:
-    h = t if isinstance(t, _HostArray) else _HostArray(t)
+    if isinstance(t, _HostArray):
+        h = t
+    else:
+        a = _host_array(t)
+        h = _HostArray(a, _content(a))
     dev = torch.device(device)
     if dev.type == "cuda" and dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
@@ -360,12 +370,24 @@ _PACKS: "collections.OrderedDict" = collections.OrderedDict()
 
 
 def _pack(cls, batch: int, device, n_proj: int, arrays, build):
-    if any(isinstance(a, torch.Tensor) and a.is_cuda for a in arrays):
-        return build(*arrays)
-    arrays = [None if a is None else _HostArray(a) for a in arrays]
-    key = (cls, batch, n_proj, device, *(a and a.key for a in arrays))
+    host, key = [], [cls, batch, n_proj, device]
+    for a in arrays:
+        if a is not None:
+            if isinstance(a, torch.Tensor):
+                if a.is_cuda:
+                    return build(*arrays)
+                a = a.detach().numpy()
+            a = np.ascontiguousarray(a, dtype=np.float32)
+            key.append(a.shape)
+            key.append(a.tobytes() if a.nbytes <= 4096 else _content(a))
+        else:
+            key.append(None)
+            key.append(None)
+        host.append(a)
+    key = tuple(key)
     hit = _PACKS.get(key)
     if hit is None:
+        arrays = [None if a is None else _HostArray(a, c) for a, c in zip(host, key[5::2])]
         if device.type == "cuda" and torch.cuda.is_current_stream_capturing():
             return build(*arrays)  # what a capture computes exists only when its graph is replayed
         hit = build(*arrays)
