@@ -1,5 +1,5 @@
 // fdk_taps.cuh -- the spatial ramp-filter kernels of the FDK / FBP filter,
-// shared by its CUDA-core and tensor-core implementations.
+// shared by its direct sums (fdk.cu, fdk_fft.cu's rows out of range).
 //
 // tau * h[m] for the Ram-Lak and Shepp-Logan kernels of Kak & Slaney (1988,
 // ch. 3), tau the detector column pitch: Ram-Lak h[0] = 1 / (4 tau^2),

@@ -51,6 +51,7 @@ constexpr long long BP2_SPLIT_MAX_PIXELS = 131072;     // pixels per launch up t
 constexpr long long BP2_SPLIT_MAX_SHARED = 600000;     // the same, threads of several slices
 constexpr long long BP2_SHARE_MIN_PIXELS = 80000;      // pixels per launch from which a thread takes several slices
 constexpr long long BP2_NS8_MIN_PIXELS = 8000000;      // pixels per launch from which a thread takes eight slices
+static_assert(BP2_NS8_MIN_PIXELS / 8 > BP2_SPLIT_MAX_SHARED, "eight slices are never split");
 
 // Two values on the packed FP32 instructions: one issue slot for both (the
 // kernels here are bound by issue).
@@ -922,17 +923,20 @@ cudaError_t bp_typed(const void *sinogram, void *volume, bool fan, const Dims2D 
     };
     auto launch_slices = [&](auto ns_c) {
         constexpr int NS = decltype(ns_c)::value;
-        if (fan && split) {  // every block runs in exactly one of the two (see the kernel)
-            launch(backprojection2d_kernel<Tin, Tout, true, false, BP2_VSPLIT, NS>);
-            launch(backprojection2d_kernel<Tin, Tout, true, true, BP2_VSPLIT, NS>);
-        } else if (fan) {
-            launch(backprojection2d_kernel<Tin, Tout, true, false, 1, NS>);
-            launch(backprojection2d_kernel<Tin, Tout, true, true, 1, NS>);
-        } else if (split) {
-            launch(backprojection2d_kernel<Tin, Tout, false, false, BP2_VSPLIT, NS>);
-        } else {
-            launch(backprojection2d_kernel<Tin, Tout, false, false, 1, NS>);
+        // (eight slices leave at least BP2_NS8_MIN_PIXELS / 8 threads: no view groups)
+        auto launch_split = [&](auto vsplit_c) {
+            constexpr int VSPLIT = decltype(vsplit_c)::value;
+            if (fan) {  // every block runs in exactly one of the two (see the kernel)
+                launch(backprojection2d_kernel<Tin, Tout, true, false, VSPLIT, NS>);
+                launch(backprojection2d_kernel<Tin, Tout, true, true, VSPLIT, NS>);
+            } else {
+                launch(backprojection2d_kernel<Tin, Tout, false, false, VSPLIT, NS>);
+            }
+        };
+        if constexpr (NS < 8) {
+            if (split) return launch_split(std::integral_constant<int, BP2_VSPLIT>{});
         }
+        launch_split(std::integral_constant<int, 1>{});
     };
     if (ns == 8)
         launch_slices(std::integral_constant<int, 8>{});

@@ -92,3 +92,21 @@ def test_filter_short_rows(cuda, width, rows, kind):
     got = out.double().cpu().numpy()
     for r in range(rows):
         assert rel_l2(got[r], ref[r]) < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("in_place", [False, True])
+@pytest.mark.parametrize("width,kind", [(48, 0), (255, 1), (2048, 0), (2049, 0), (2049, 1), (3000, 1), (4096, 0)])
+def test_filter_in_place_and_types(cuda, width, kind, in_place, dtype):
+    """Ordinary rows of every storage type, filtered in place and not, by
+    transforms and (above 2048) by direct sums: 1e-5, and half an ulp of 16-bit
+    outputs."""
+    p = np.random.Generator(np.random.PCG64(width)).uniform(0.2, 1.0, (5, width))
+    x = torch.as_tensor(p, dtype=dtype, device=cuda)
+    ref, _ = _direct(x.double().cpu().numpy(), kind)
+    out = x if in_place else torch.empty_like(x)
+    code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
+    _capi.call("pyronn_fdk_filter", x.data_ptr(), out.data_ptr(), code, code, 1, 1, 5, width, SDD, DV, DU, 2.0,
+               (width - 1) / 2, kind, 0, torch.cuda.current_stream().cuda_stream)
+    rounding = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -11}[dtype]
+    assert rel_l2(out.double().cpu().numpy(), ref) < 1e-5 + rounding
