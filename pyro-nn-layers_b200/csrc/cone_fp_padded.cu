@@ -8,9 +8,10 @@
 // sample at nearly the same (x, y) and at consecutive z whenever the
 // detector's v axis runs along z -- true for every view of a circular
 // trajectory.  Such views ("z mode") lay warps along v and read a z-fastest
-// copy of trilinear CELLS: the element of cell (x, y, z) holds all eight taps
-// V(x + {0,1}, y + {0,1}, z + {0,1}), so a sample is ONE 16-byte load (two
-// for FP32) whose warp-wide footprint is a few consecutive lines.
+// copy of trilinear CELLS: the element of cell (x, y, z) holds the eight taps
+// V(x + {0,1}, y + {0,1}, z + {0,1}) of a 16-bit volume, the four at z of an FP32
+// one, so a sample is ONE 16-byte load (FP32: two adjacent ones) whose
+// warp-wide footprint is a few consecutive lines.
 // Other views ("xy mode") lay warps along u and read an x-fastest or a
 // y-fastest copy, whichever fastest axis runs across their rays.
 // All copies carry a zero border, so the taps of any sample inside the box
