@@ -1,5 +1,7 @@
 """Cached geometry outlives the work that reads it, on whatever stream, and
 dropping an entry waits for nothing."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -88,3 +90,37 @@ def test_eviction_beside_a_busy_stream(cuda, backward):
     assert not side.query(), "dropping geometry waited for another stream"
     torch.cuda.synchronize()
     assert torch.equal(got, want) and all(bool(torch.isnan(j).all()) for j in junk)
+
+
+@pytest.mark.gpu
+def test_threads_share_the_caches(cuda):
+    """Threads with a stream each, over more geometry than the caches hold: each
+    call's result is that of the call alone."""
+    x = torch.rand((1, 24, 24, 24), device=cuda)
+    geos = [_geo(300 + k) for k in range(ops._HOST_GEOM_CACHE_SIZE + 16)]
+
+    def project(k):
+        return pl.cone_projection3d(x, geos[k].detector_shape, *geos[k].args())
+
+    want = [project(k) for k in range(len(geos))]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(seed):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                order = np.random.Generator(np.random.PCG64(seed)).permutation(np.repeat(np.arange(len(geos)), 3))
+                got = [(int(k), project(int(k))) for k in order]
+                stream.synchronize()
+                assert all(torch.equal(y, want[k]) for k, y in got)
+                stream.synchronize()
+        except BaseException as e:  # reported by the test's own thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(120)
+    assert not errors and not any(t.is_alive() for t in threads)
